@@ -159,6 +159,20 @@ __device__ __forceinline__ int wrap_axis(int u, int n, int periodic, int& side) 
   return u < n ? u : u % n;
 }
 
+// The same without branches, for the one-thread-per-point kernels: an index
+// that is always inside the array (0 for a zero point) and whether there is a
+// value at all (ok).  At most one wrap, which their outputs need.  A thread's
+// loads then do not depend on one another's range checks and are all in
+// flight together; with a branch per neighbour they were taken one after the
+// other, about 0.6 us each.
+__device__ __forceinline__ int map_axis(int u, int n, int periodic, int& side, bool& ok) {
+  const bool in = unsigned(u) < unsigned(n);
+  const int w = u < 0 ? u + n : u - n;
+  ok = in || periodic;
+  side = in || !periodic ? -1 : (u < 0 ? 1 : 0);
+  return in ? u : (periodic ? w : 0);
+}
+
 // The same for a plane index of a marching kernel, which lies in
 // [-R, n + R) with n >= R on a periodic axis: one wrap at most.
 __device__ __forceinline__ int wrap_plane(int u, int n, int periodic, int& side) {
@@ -182,6 +196,28 @@ struct Phases {
 template <class S>
 __device__ __forceinline__ cplx<S> phase_of(const Phases<S>& P, int c, int side) {
   return P.ph[c][side];
+}
+
+// v times the phase of axis c's wrapped side (side < 0: v itself), without a
+// branch.
+template <class V, class S>
+__device__ __forceinline__ V side_phase(const Phases<S>& P, int c, int side, V v) {
+  if constexpr (vt<V>::NC == 2) {
+    const cplx<S> ph = {side == 1 ? P.ph[c][1].re : P.ph[c][0].re,
+                        side == 1 ? P.ph[c][1].im : P.ph[c][0].im};
+    const V w = cmul(ph, v);
+    v.re = side >= 0 ? w.re : v.re;
+    v.im = side >= 0 ? w.im : v.im;
+  }
+  return v;
+}
+
+// A value where ok, zero elsewhere (a select, not a product).
+__device__ __forceinline__ double value_or_zero(bool ok, double v) { return ok ? v : 0.0; }
+__device__ __forceinline__ float value_or_zero(bool ok, float v) { return ok ? v : 0.0f; }
+template <class S>
+__device__ __forceinline__ cplx<S> value_or_zero(bool ok, const cplx<S>& v) {
+  return {ok ? v.re : S(0), ok ? v.im : S(0)};
 }
 
 // ---------------------------------------------------------------------------

@@ -57,7 +57,7 @@ struct GStar {
 };
 struct GGs {
   GHead h;
-  GenParams<double> p;
+  StarParams<double> p;
   double* phi;
   const double* rho;
   const double* frozen;
@@ -151,11 +151,12 @@ g_star_kernel(const GStar* __restrict__ items, int nitems, int ntiles, unsigned*
 }
 
 // One colour of multicolour Gauss-Seidel.
+template <int R>
 __global__ void __launch_bounds__(kGThreads)
 g_gs_kernel(const GGs* __restrict__ items, int nitems, int ntiles, unsigned* ctr,
             const int* __restrict__ active, int ncolor, int color) {
   pdl_enter();
-  __shared__ __align__(16) GenParams<double> sp;
+  __shared__ __align__(16) StarParams<double> sp;
   int t, i;
   while (next_tile(items, nitems, ntiles, ctr, t, i)) {
     const GGs& it = items[i];
@@ -170,7 +171,7 @@ g_gs_kernel(const GGs* __restrict__ items, int nitems, int ntiles, unsigned* ctr
       if (q >= nq) break;
       int i0, i1, i2;
       if (gs_colour_point(q, slots, ncolor, color, sp.n1, sp.n2, i0, i1, i2))
-        gs_point_at<double>(it.phi, it.rho, it.frozen, sp, i0, i1, i2);
+        gs_star_point_at<double, R>(it.phi, it.rho, it.frozen, sp, i0, i1, i2);
     }
   }
 }
@@ -265,7 +266,8 @@ g_check_kernel(SolveCtrl* const* ctrl, int* active, const int* tile0, const int*
   if (threadIdx.x == 0) cudaGraphSetConditional(loop, any ? 1u : 0u);
 }
 
-enum { S_JACOBI, S_RESID, S_RESID_NORM, S_GS, S_RESTRICT, S_INTERP, S_FILL };
+// S_GS + R: a Gauss-Seidel colour of a radius-R stencil.
+enum { S_JACOBI, S_RESID, S_RESID_NORM, S_RESTRICT, S_INTERP, S_FILL, S_GS };
 
 struct Step {
   int kind;
@@ -341,11 +343,11 @@ void relax_steps(PoissonGroup* G, int l, int& cur, int nsweeps) {
           return it;
         });
       for (int color = 0; color < nc; color++)
-        add_step<GGs>(G, S_GS, nc, color, [&](int i) {
+        add_step<GGs>(G, S_GS + op0->R, nc, color, [&](int i) {
           const Level& lv = G->ps[i]->L[l];
           GGs it{};
           it.h.n = (long long)lv.op->n[0] * lv.op->n[1] * gs_row_slots(lv.op->n[2], nc);
-          gs_params(lv.op, it.p);
+          gs_star_params(lv.op, it.p);
           it.phi = dptr(lv.phi[c]);
           it.rho = dptr(lv.rho);
           it.frozen = any_per ? dptr(lv.phi[1 - c]) : dptr(lv.phi[c]);
@@ -466,6 +468,14 @@ int launch_star_step(const PoissonGroup* G, const Step& st, int k, cudaStream_t 
   return check_launch("g_star_kernel");
 }
 
+template <int R>
+int launch_gs_step(const PoissonGroup* G, const Step& st, int k, cudaStream_t s) {
+  launch_k(g_gs_kernel<R>, step_blocks(st), kGThreads, 0, s,
+           reinterpret_cast<const GGs*>(G->d_items + st.off), st.nitems, st.ntiles, G->d_ctr + k,
+           (const int*)G->d_active, st.a, st.b);
+  return check_launch("g_gs_kernel");
+}
+
 template <int NN>
 int launch_tr_step(const PoissonGroup* G, const Step& st, int k, cudaStream_t s) {
   const GTr* items = reinterpret_cast<const GTr*>(G->d_items + st.off);
@@ -493,11 +503,12 @@ int launch_step(const PoissonGroup* G, int k, cudaStream_t s) {
         case 6: return launch_star_step<6>(G, st, k, s);
       }
       return set_error(GFD_EUNSUPPORTED, "stencil radius out of range");
-    case S_GS:
-      launch_k(g_gs_kernel, step_blocks(st), kGThreads, 0, s,
-               reinterpret_cast<const GGs*>(G->d_items + st.off), st.nitems, st.ntiles,
-               G->d_ctr + k, (const int*)G->d_active, st.a, st.b);
-      return check_launch("g_gs_kernel");
+    case S_GS + 1: return launch_gs_step<1>(G, st, k, s);
+    case S_GS + 2: return launch_gs_step<2>(G, st, k, s);
+    case S_GS + 3: return launch_gs_step<3>(G, st, k, s);
+    case S_GS + 4: return launch_gs_step<4>(G, st, k, s);
+    case S_GS + 5: return launch_gs_step<5>(G, st, k, s);
+    case S_GS + 6: return launch_gs_step<6>(G, st, k, s);
     case S_RESTRICT:
     case S_INTERP:
       switch (st.a) {

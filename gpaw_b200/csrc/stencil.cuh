@@ -454,33 +454,25 @@ __device__ __forceinline__ V star_point_at(const V* __restrict__ base, const V* 
                                            const StarParams<typename vt<V>::S>& p, int i0, int i1,
                                            int i2, long long rem) {
   using Sc = typename vt<V>::S;
-  const long long plane = (long long)p.n1 * p.n2;
-  const int r1 = int(rem - i0 * plane);
   Sc cc = p.c0;
   if constexpr (MODE == MODE_POTENTIAL) cc += LD::ld(static_cast<const Sc*>(p.pot) + rem);
   V s = vmul(cc, LD::ld(base + rem));
+  // 32-bit offsets: a band holds fewer than 2^27 points.
+  const int pl = p.n1 * p.n2, row = i0 * pl + i1 * p.n2, ownr = int(rem);
 #pragma unroll
   for (int k = -R; k <= R; k++) {
     if (k == 0) continue;
     int sd;
-    int j = wrap_axis(i0 + k, p.n0, p.per0, sd);
-    if (j >= 0) {
-      V v = LD::ld(base + j * plane + r1);
-      if constexpr (vt<V>::NC == 2) { if (sd >= 0) v = phase_mul(phase_of(p.P, 0, sd), v); }
-      madd(s, p.cx[kMaxR + k], v);
-    }
-    j = wrap_axis(i1 + k, p.n1, p.per1, sd);
-    if (j >= 0) {
-      V v = LD::ld(base + i0 * plane + j * p.n2 + i2);
-      if constexpr (vt<V>::NC == 2) { if (sd >= 0) v = phase_mul(phase_of(p.P, 1, sd), v); }
-      madd(s, p.cy[kMaxR + k], v);
-    }
-    j = wrap_axis(i2 + k, p.n2, p.per2, sd);
-    if (j >= 0) {
-      V v = LD::ld(base + i0 * plane + i1 * p.n2 + j);
-      if constexpr (vt<V>::NC == 2) { if (sd >= 0) v = phase_mul(phase_of(p.P, 2, sd), v); }
-      madd(s, p.cz[kMaxR + k], v);
-    }
+    bool ok;
+    int j = map_axis(i0 + k, p.n0, p.per0, sd, ok);
+    V v = value_or_zero(ok, LD::ld(base + (j * pl + (ownr - i0 * pl))));
+    madd(s, p.cx[kMaxR + k], side_phase(p.P, 0, sd, v));
+    j = map_axis(i1 + k, p.n1, p.per1, sd, ok);
+    v = value_or_zero(ok, LD::ld(base + (i0 * pl + j * p.n2 + i2)));
+    madd(s, p.cy[kMaxR + k], side_phase(p.P, 1, sd, v));
+    j = map_axis(i2 + k, p.n2, p.per2, sd, ok);
+    v = value_or_zero(ok, LD::ld(base + (row + j)));
+    madd(s, p.cz[kMaxR + k], side_phase(p.P, 2, sd, v));
   }
   if constexpr (MODE == MODE_JACOBI) return vmul(p.wc, vsub(LD::ld(rho_b + rem), s));
   else if constexpr (MODE == MODE_RESIDUAL) return vsub(s, LD::ld(rho_b + rem));
@@ -664,6 +656,36 @@ __device__ __forceinline__ void gs_point_at(V* phi, const V* __restrict__ rho, c
   phi[g] = (rho[g] - s) * (S(1) / p.coefs[0]);
 }
 
+// The same for an axis-aligned stencil of radius R (p.c0 the diagonal, p.wc
+// its reciprocal).  Every neighbour's load is independent, so the update
+// costs about one memory round trip; the loop over an offset table above
+// pays one per neighbour.
+template <class V, int R>
+__device__ __forceinline__ void gs_star_point_at(V* phi, const V* __restrict__ rho, const V* frozen,
+                                                 const StarParams<typename vt<V>::S>& p, int i0,
+                                                 int i1, int i2) {
+  using S = typename vt<V>::S;
+  static_assert(vt<V>::NC == 1, "Gauss-Seidel works on real arrays");
+  const int pl = p.n1 * p.n2, row = i0 * pl + i1 * p.n2, g = row + i2;
+  S sx = 0, sy = 0, sz = 0;
+#pragma unroll
+  for (int k = -R; k <= R; k++) {
+    if (k == 0) continue;
+    int sd;
+    bool ok;
+    int j = map_axis(i0 + k, p.n0, p.per0, sd, ok);
+    const V vx = value_or_zero(ok, (sd >= 0 ? frozen : phi)[j * pl + (g - i0 * pl)]);
+    j = map_axis(i1 + k, p.n1, p.per1, sd, ok);
+    const V vy = value_or_zero(ok, (sd >= 0 ? frozen : phi)[i0 * pl + j * p.n2 + i2]);
+    j = map_axis(i2 + k, p.n2, p.per2, sd, ok);
+    const V vz = value_or_zero(ok, (sd >= 0 ? frozen : phi)[row + j]);
+    madd(sx, p.cx[kMaxR + k], vx);
+    madd(sy, p.cy[kMaxR + k], vy);
+    madd(sz, p.cz[kMaxR + k], vz);
+  }
+  phi[g] = (rho[g] - (sx + (sy + sz))) * p.wc;
+}
+
 // Points of one colour, enumerated without idle threads: index q covers
 // the rows (i0, i1) times gs_row_slots() slots; slot j of a row is
 // i2 = first + ncolor j, first = (color - i0 - i1) mod ncolor.  False for
@@ -694,6 +716,20 @@ color_gs_kernel(V* phi, const V* __restrict__ rho, const V* frozen,
     int i0, i1, i2;
     if (gs_colour_point(q, slots, ncolor, color, p.n1, p.n2, i0, i1, i2))
       gs_point_at<V>(phi, rho, frozen, p, i0, i1, i2);
+  }
+}
+
+template <class V, int R>
+__global__ void __launch_bounds__(256)
+color_gs_star_kernel(V* phi, const V* __restrict__ rho, const V* frozen,
+                     const StarParams<typename vt<V>::S> p, int ncolor, int color) {
+  pdl_enter();
+  const int slots = gs_row_slots(p.n2, ncolor);
+  const int nq = p.n0 * p.n1 * slots;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
+    int i0, i1, i2;
+    if (gs_colour_point(q, slots, ncolor, color, p.n1, p.n2, i0, i1, i2))
+      gs_star_point_at<V, R>(phi, rho, frozen, p, i0, i1, i2);
   }
 }
 

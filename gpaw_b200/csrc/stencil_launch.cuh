@@ -588,12 +588,17 @@ void gs_params(const gfd_operator* op, GenParams<S>& p) {
   }
 }
 
-template <class V>
-int gs_typed(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* frozen, int ncolor,
-             cudaStream_t s) {
-  using S = typename vt<V>::S;
-  GenParams<S> p;
-  gs_params(op, p);
+// The same for an axis-aligned stencil (gs_star_point_at).
+template <class S>
+void gs_star_params(const gfd_operator* op, StarParams<S>& p) {
+  star_params(op, OP_APPLY, 0.0, nullptr, p);
+  p.wc = S(1) / p.c0;
+}
+
+// Gauss-Seidel sweeps: one launch per colour, R = 0 for offset tables.
+template <class V, int R, class P>
+int gs_sweeps(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* frozen, int ncolor,
+              const P& p, cudaStream_t s) {
   const long long n = p.band;
   const bool any_per = op->per[0] || op->per[1] || op->per[2];
   const long long nq = (long long)op->n[0] * op->n[1] * gs_row_slots(op->n[2], ncolor);
@@ -603,10 +608,36 @@ int gs_typed(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* froze
       cudaError_t e = cudaMemcpyAsync(frozen, phi, n * sizeof(V), cudaMemcpyDeviceToDevice, s);
       if (e != cudaSuccess) return check_cuda(e, "cudaMemcpyAsync(frozen)");
     }
-    for (int c = 0; c < ncolor; c++)
-      launch_k(color_gs_kernel<V>, blocks, 256, 0, s, phi, rho, any_per ? frozen : phi, p, ncolor, c);
+    V* fr = any_per ? frozen : phi;
+    for (int c = 0; c < ncolor; c++) {
+      if constexpr (R == 0)
+        launch_k(color_gs_kernel<V>, blocks, 256, 0, s, phi, rho, fr, p, ncolor, c);
+      else
+        launch_k(color_gs_star_kernel<V, R>, blocks, 256, 0, s, phi, rho, fr, p, ncolor, c);
+    }
   }
   return check_launch("color_gs_kernel");
+}
+
+template <class V>
+int gs_typed(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* frozen, int ncolor,
+             cudaStream_t s) {
+  using S = typename vt<V>::S;
+  if (op->star) {
+    StarParams<S> p;
+    gs_star_params(op, p);
+    switch (op->R) {
+      case 1: return gs_sweeps<V, 1>(op, phi, rho, nsweeps, frozen, ncolor, p, s);
+      case 2: return gs_sweeps<V, 2>(op, phi, rho, nsweeps, frozen, ncolor, p, s);
+      case 3: return gs_sweeps<V, 3>(op, phi, rho, nsweeps, frozen, ncolor, p, s);
+      case 4: return gs_sweeps<V, 4>(op, phi, rho, nsweeps, frozen, ncolor, p, s);
+      case 5: return gs_sweeps<V, 5>(op, phi, rho, nsweeps, frozen, ncolor, p, s);
+      case 6: return gs_sweeps<V, 6>(op, phi, rho, nsweeps, frozen, ncolor, p, s);
+    }
+  }
+  GenParams<S> p;
+  gs_params(op, p);
+  return gs_sweeps<V, 0>(op, phi, rho, nsweeps, frozen, ncolor, p, s);
 }
 
 }  // namespace gfd

@@ -462,33 +462,67 @@ interp_kernel(const V* __restrict__ in, V* out, const V* base,
 // the L1 cache.  The marching kernels above pay a memory round trip per plane,
 // which dominates on grids of a few thousand points.
 // ---------------------------------------------------------------------------
+// Input position u of an axis: element offset (always inside the band) in
+// units of the axis stride, whether it holds a value, and its wrap side.
+struct TrTap {
+  int off;
+  int side;
+  bool ok;
+};
+__device__ __forceinline__ TrTap tr_map(int u, int n, int per, int stride) {
+  TrTap t;
+  t.off = map_axis(u, n, per, t.side, t.ok) * stride;
+  return t;
+}
 template <class LD, class V, class S>
-__device__ __forceinline__ V tr_fetch(const V* base, int x, int y, int z, const TrParams<S>& p) {
-  int sx, sy, sz;
-  const int i = wrap_axis(x, p.ni0, p.per0, sx);
-  const int j = wrap_axis(y, p.ni1, p.per1, sy);
-  const int k = wrap_axis(z, p.ni2, p.per2, sz);
-  if (i < 0 || j < 0 || k < 0) return vzero<V>();
-  V v = LD::ld(base + ((long long)i * p.ni1 + j) * p.ni2 + k);
+__device__ __forceinline__ V tr_fetch(const V* base, const TrTap& x, const TrTap& y,
+                                      const TrTap& z, const TrParams<S>& p) {
+  V v = value_or_zero(x.ok && y.ok && z.ok, LD::ld(base + (x.off + y.off + z.off)));
   if constexpr (vt<V>::NC == 2) {
-    if (sx >= 0) v = phase_mul(phase_of(p.P, 0, sx), v);
-    if (sy >= 0) v = phase_mul(phase_of(p.P, 1, sy), v);
-    if (sz >= 0) v = phase_mul(phase_of(p.P, 2, sz), v);
+    v = side_phase(p.P, 0, x.side, v);
+    v = side_phase(p.P, 1, y.side, v);
+    v = side_phase(p.P, 2, z.side, v);
   }
   return v;
 }
 
+// rst_tap with the pairs in a loop (not unrolled): the outer axes of the
+// wider transfers, whose (2nn + 1)^3 taps would otherwise all be expanded.
+template <int NN, class V, class Get>
+__device__ __forceinline__ V rst_tap_loop(Get get) {
+  using S = typename vt<V>::S;
+  if constexpr (NN == 1) {
+    return rst_tap<NN, V>(get);
+  } else {
+    V x = get(0);
+#pragma unroll 1
+    for (int k = 0; k < NN; k++)
+      x = vadd(x, vmul(lagw<NN, S>(k), vadd(get(2 * k + 1), get(-(2 * k + 1)))));
+    return vmul(S(0.5), x);
+  }
+}
+
 // One restricted point at output coordinates (X, Y, Z) of a band (base:
 // the band's input), times out_scale; LD is the load policy (common.cuh).
+// The axis-2 taps (all 27 taps for nn = 1) are loaded without branches, so
+// they are in flight together.
 template <class V, int NN, class LD>
 __device__ __forceinline__ V restrict_point_at(const V* __restrict__ base, int X, int Y, int Z,
                                                const TrParams<typename vt<V>::S>& p) {
   constexpr int W = 2 * NN - 1;
   // fine centre of each axis: 2i + (2nn-1) - lo
   const int fx = 2 * X + W - p.lo0, fy = 2 * Y + W - p.lo1, fz = 2 * Z + W - p.lo2;
-  V v = rst_tap<NN, V>([&](int ox) {
-    return rst_tap<NN, V>([&](int oy) {
-      return rst_tap<NN, V>([&](int oz) { return tr_fetch<LD>(base, fx + ox, fy + oy, fz + oz, p); });
+  TrTap tz[2 * NN + 1];  // slot (o + W) / 2 for the odd offsets, 2nn the centre
+#pragma unroll
+  for (int j = 0; j < 2 * NN; j++) tz[j] = tr_map(fz - W + 2 * j, p.ni2, p.per2, 1);
+  tz[2 * NN] = tr_map(fz, p.ni2, p.per2, 1);
+  V v = rst_tap_loop<NN, V>([&](int ox) {
+    const TrTap tx = tr_map(fx + ox, p.ni0, p.per0, p.ni1 * p.ni2);
+    return rst_tap_loop<NN, V>([&](int oy) {
+      const TrTap ty = tr_map(fy + oy, p.ni1, p.per1, p.ni2);
+      return rst_tap<NN, V>([&](int oz) {
+        return tr_fetch<LD>(base, tx, ty, tz[oz == 0 ? 2 * NN : (oz + W) >> 1], p);
+      });
     });
   });
   if (p.out_scale != typename vt<V>::S(1)) v = vmul(p.out_scale, v);
@@ -508,8 +542,25 @@ __device__ __forceinline__ V restrict_point(const V* __restrict__ in,
   return restrict_point_at<V, NN, LD>(in + b * p.band_in, X, Y, Z, p);
 }
 
+// A value where even, the K-tap value of `get` where odd; both are computed
+// for nn = 1 (a select, so no lane waits for another's path), the wider taps
+// branch.
+template <int NN, class V, class Get>
+__device__ __forceinline__ V ip_along(int odd, Get get) {
+  if constexpr (NN == 1) {
+    const V a = get(0), m = ip_tap<NN, V>([&](int o) { return o == 0 ? a : get(odd); });
+    V r;
+    if constexpr (vt<V>::NC == 2) r = {odd ? m.re : a.re, odd ? m.im : a.im};
+    else r = odd ? m : a;
+    return r;
+  } else {
+    return odd ? ip_tap<NN, V>(get) : get(0);
+  }
+}
+
 // One interpolated point at output coordinates (X, Y, Z), times out_scale
-// (SUB: *bo, the base value at that point, minus it).
+// (SUB: *bo, the base value at that point, minus it).  For nn = 1 the eight
+// corner loads are independent (an even axis reads its one point twice).
 template <class V, int NN, bool SUB, class LD>
 __device__ __forceinline__ V interp_point_at(const V* __restrict__ base, const V* bo, int X, int Y,
                                              int Z, const TrParams<typename vt<V>::S>& p) {
@@ -517,15 +568,20 @@ __device__ __forceinline__ V interp_point_at(const V* __restrict__ base, const V
   const int gx = X + p.sk0, gy = Y + p.sk1, gz = Z + p.sk2;
   const int cx = (gx >> 1) + NN - 1 - p.lo0, cy = (gy >> 1) + NN - 1 - p.lo1,
             cz = (gz >> 1) + NN - 1 - p.lo2;
-  auto along = [&](int odd, auto get) -> V { return odd ? ip_tap<NN, V>(get) : get(0); };
-  V v = along(gx & 1, [&](int ox) {
-    return along(gy & 1, [&](int oy) {
-      return along(gz & 1, [&](int oz) { return tr_fetch<LD>(base, cx + ox, cy + oy, cz + oz, p); });
+  V b = vzero<V>();
+  // bo may be the output itself (in-place correction): a plain load.
+  if constexpr (SUB) b = *bo;
+  V v = ip_along<NN, V>(gx & 1, [&](int ox) {
+    const TrTap tx = tr_map(cx + ox, p.ni0, p.per0, p.ni1 * p.ni2);
+    return ip_along<NN, V>(gy & 1, [&](int oy) {
+      const TrTap ty = tr_map(cy + oy, p.ni1, p.per1, p.ni2);
+      return ip_along<NN, V>(gz & 1, [&](int oz) {
+        return tr_fetch<LD>(base, tx, ty, tr_map(cz + oz, p.ni2, p.per2, 1), p);
+      });
     });
   });
   if (p.out_scale != typename vt<V>::S(1)) v = vmul(p.out_scale, v);
-  // bo may be the output itself (in-place correction): a plain load.
-  if constexpr (SUB) v = vsub(*bo, v);
+  if constexpr (SUB) v = vsub(b, v);
   return v;
 }
 

@@ -214,6 +214,24 @@ BLOCKED_SHAPES = [((24, 16, 33), 1), ((40, 20, 36), 1), ((40, 20, 36), 0), ((17,
                   ((9, 33, 64), (1, 1, 0))]
 
 
+@pytest.mark.parametrize('n,nn,pbc', [((3, 3, 3), 3, True), ((5, 4, 7), 2, (True, False, True)),
+                                      ((2, 2, 2), 3, False), ((9, 6, 13), 4, True),
+                                      ((33, 17, 12), 1, False)])
+def test_gauss_seidel_radii_and_edges(cuda, n, nn, pbc):
+    """Colour passes of axis-aligned stencils of each radius on grids down to
+    the stencil's reach, one sweep, against the colour-by-colour reference.
+    One sweep divides once by the diagonal: 1e-13 as for the stencils."""
+    from gpaw_b200.fd_operators import FDOperator
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    gd = GridDescriptor(n, tuple(0.3 * x for x in n), pbc)
+    c, o = G.laplace_stencil(G.Grid(n, tuple(0.3 * x for x in n), pbc), -0.25 / np.pi, nn)
+    rng = np.random.RandomState(4)
+    phi0, rho = (rng.standard_normal(tuple(gd.n_c)) for _ in range(2))
+    phi = dev(phi0, cuda)
+    FDOperator(c, o, gd, float).relax(1, phi, dev(rho, cuda), 1)
+    assert rel_err(host(phi), multicolour_gs_reference(c, o, gd.pbc_c, phi0, rho, 1)) < TOL
+
+
 @pytest.mark.parametrize('N,pbc', BLOCKED_SHAPES)
 @pytest.mark.parametrize('n', [1, 2, 3])
 def test_register_blocked_tiles(cuda, N, pbc, n):

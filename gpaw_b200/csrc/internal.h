@@ -24,6 +24,9 @@ struct gfd_operator {
   double c0 = 0.0;
   double cx[13] = {0}, cy[13] = {0}, cz[13] = {0};  // index 6 + k
   double diag = 0.0;     // weight of the zero offset
+  // Every offset is k d with d one of the 13 lattice directions (every
+  // component -1, 0 or 1) or their opposites: dirs_kernel's class.
+  bool dirs = false;
   // Device scratch of one grid for relaxation (Jacobi ping-pong / frozen
   // copy for periodic Gauss-Seidel), allocated on first use.
   void* scratch = nullptr;

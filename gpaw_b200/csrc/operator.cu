@@ -349,6 +349,15 @@ extern "C" int gfd_operator_create(int ncoefs, const double* coefs, const int64_
   for (int c = 0; c < ncoefs; c++)
     if (op->off[3 * c] == 0 && op->off[3 * c + 1] == 0 && op->off[3 * c + 2] == 0)
       op->diag = coefs[c];
+  op->dirs = mp >= 1;
+  for (int c = 0; c < ncoefs; c++) {
+    int m = 0;
+    for (int a = 0; a < 3; a++) m = std::max(m, std::abs(op->off[3 * c + a]));
+    for (int a = 0; a < 3; a++) {
+      const int o = std::abs(op->off[3 * c + a]);
+      if (o != 0 && o != m) op->dirs = false;
+    }
+  }
   // Axis-aligned decomposition.
   bool star = mp <= kMaxR;
   for (int c = 0; c < ncoefs && star; c++) {

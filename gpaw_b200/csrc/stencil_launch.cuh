@@ -8,6 +8,7 @@
 
 #include "internal.h"
 #include "stencil.cuh"
+#include "stencil_dirs.cuh"
 #include "stencil_split.cuh"
 #include "stencil_tma.cuh"
 #include "stencil_tmasplit.cuh"
@@ -501,6 +502,126 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
   return star_dispatch<V, MODE_APPLY>(op, tile, vin, vout, nullptr, nin, p, g, nullptr, s);
 }
 
+// ---------------------------------------------------------------------------
+// Lattice-direction stencils (stencil_dirs.cuh): 256 threads, 2 rows each, two
+// CTAs per SM; tile sides fit the grid (bz columns up to 48, the rows that the
+// threads and 110 KB of staged 16-byte cells allow).
+// ---------------------------------------------------------------------------
+constexpr int kDirNT = 256, kDirVY = 2, kDirBZ = 48, kDirCPT = 5, kDirStages = 4;
+constexpr size_t kDirSmem = 110 * 1024;
+
+inline bool dirs_eligible(const gfd_operator* op, int mode) {
+  return op->dirs && op->mp <= (mode == OP_APPLY ? kDirMaxR : 3);
+}
+
+struct DirGeom {
+  int bz, ty, gx, gy, nxc, x_chunk;
+  int64_t bands_per_launch;
+};
+inline DirGeom dirs_geom(const gfd_operator* op, int64_t nin) {
+  const int R = op->mp;
+  DirGeom g;
+  g.gx = (op->n[2] + kDirBZ - 1) / kDirBZ;
+  g.bz = (op->n[2] + g.gx - 1) / g.gx;
+  auto fits = [&](int ty) {
+    const int rows = ty * kDirVY + 2 * R;
+    return (g.bz + 2 * R) * rows <= kDirCPT * kDirNT &&
+           size_t(kDirStages) * rows * (kDirBZ + 2 * R) * 16 <= kDirSmem;
+  };
+  int ty = kDirNT / g.bz;
+  while (ty > 1 && !fits(ty)) ty--;
+  g.gy = (op->n[1] + ty * kDirVY - 1) / (ty * kDirVY);
+  const int rows = (op->n[1] + g.gy - 1) / g.gy;
+  g.ty = (rows + kDirVY - 1) / kDirVY;
+  g.gy = (op->n[1] + g.ty * kDirVY - 1) / (g.ty * kDirVY);
+  const int64_t tiles = (int64_t)g.gx * g.gy * std::max<int64_t>(nin, 1);
+  const int64_t target = 4LL * num_sms();
+  const int maxc = std::max(1, op->n[0] / std::max(4, 2 * R));
+  const int nxc =
+      (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles));
+  g.x_chunk = (op->n[0] + nxc - 1) / nxc;
+  g.nxc = (op->n[0] + g.x_chunk - 1) / g.x_chunk;
+  g.bands_per_launch = std::max<int64_t>(1, 65535 / g.nxc);
+  return g;
+}
+
+template <class S>
+void dirs_params(const gfd_operator* op, int mode, double w, const double* phase_cd,
+                 const DirGeom& g, DirParams<S>& p) {
+  p = DirParams<S>{};
+  p.n0 = op->n[0]; p.n1 = op->n[1]; p.n2 = op->n[2];
+  p.per0 = op->per[0]; p.per1 = op->per[1]; p.per2 = op->per[2];
+  p.band = (long long)op->n[0] * op->n[1] * op->n[2];
+  p.bz = g.bz; p.ty = g.ty; p.x_chunk = g.x_chunk; p.nxc = g.nxc;
+  const bool jacobi = mode == OP_JACOBI || mode == OP_JACOBI_NEG;
+  double wx[2 * kDirMaxR + 1] = {0}, wh[8][kDirMaxR][3] = {};
+  for (int c = 0; c < op->ncoefs; c++) {
+    const int dx = op->off[3 * c], dy = op->off[3 * c + 1], dz = op->off[3 * c + 2];
+    double x = op->coefs[c];
+    // (1 - w) phi folded into the diagonal, as in star_kernel
+    if (jacobi && c == 0) x = -(1.0 - w) * x / w;
+    if (dy == 0 && dz == 0) {
+      wx[kDirMaxR + dx] += x;
+      continue;
+    }
+    const int k = std::max(std::abs(dy), std::abs(dz));
+    int h = 0;
+    while (half_a(h) * k != dy || half_b(h) * k != dz) ++h;
+    const int i = dx == 0 ? 0 : (dx > 0 ? 1 : 2);
+    wh[h][k - 1][i] += x;
+    p.mask |= 1u << (3 * h + i);
+  }
+  for (int i = 0; i < 2 * kDirMaxR + 1; i++) p.wx[i] = S(wx[i]);
+  for (int h = 0; h < 8; h++)
+    for (int k = 0; k < kDirMaxR; k++)
+      for (int i = 0; i < 3; i++) p.w[h][k][i] = S(wh[h][k][i]);
+  if (jacobi) {
+    p.wc = S(w / op->coefs[0]);
+    if (mode == OP_JACOBI_NEG) p.wc = -p.wc;
+  }
+  fill_phases(p.P, phase_cd);
+  if (phase_cd)
+    for (int c = 1; c < 3; c++)
+      for (int d = 0; d < 2; d++)
+        if (op->per[c] && (phase_cd[4 * c + 2 * d] != 1.0 || phase_cd[4 * c + 2 * d + 1] != 0.0))
+          p.fix_yz = 1;
+}
+
+template <class V, int R, int MODE>
+int dirs_go(const gfd_operator* op, const V* in, V* out, const V* rho, int64_t nin,
+            DirParams<typename vt<V>::S>& p, const DirGeom& g, double* partials,
+            cudaStream_t s) {
+  auto kern = dirs_kernel<V, R, kDirVY, kDirNT, 2, kDirBZ, kDirCPT, kDirStages, MODE>;
+  const size_t smem = dirs_smem_bytes<V, R, kDirVY, kDirNT, kDirBZ, kDirStages>(g.ty);
+  int st = raise_smem_limit(kern, smem, "cudaFuncSetAttribute(dirs_kernel)");
+  if (st) return st;
+  for (int64_t b0 = 0; b0 < nin; b0 += g.bands_per_launch) {
+    const int64_t nb = std::min<int64_t>(g.bands_per_launch, nin - b0);
+    p.partials = partials ? partials + b0 * g.nxc * g.gx * g.gy : nullptr;
+    launch_k(kern, dim3(g.gx, g.gy, (unsigned)(nb * g.nxc)), kDirNT, smem, s, in + b0 * p.band,
+             out + b0 * p.band, rho ? rho + b0 * p.band : nullptr, p);
+  }
+  return check_launch("dirs_kernel");
+}
+
+template <class V, int MODE>
+int dirs_dispatch(const gfd_operator* op, int mode, const V* in, V* out, const V* rho,
+                  int64_t nin, const double* phase_cd, double w, double* partials,
+                  cudaStream_t s) {
+  const DirGeom g = dirs_geom(op, nin);
+  DirParams<typename vt<V>::S> p;
+  dirs_params(op, mode, w, phase_cd, g, p);
+  switch (op->mp) {
+    case 1: return dirs_go<V, 1, MODE>(op, in, out, rho, nin, p, g, partials, s);
+    case 2: return dirs_go<V, 2, MODE>(op, in, out, rho, nin, p, g, partials, s);
+    case 3: return dirs_go<V, 3, MODE>(op, in, out, rho, nin, p, g, partials, s);
+    case 4:
+      if constexpr (MODE == MODE_APPLY)
+        return dirs_go<V, 4, MODE>(op, in, out, rho, nin, p, g, partials, s);
+  }
+  return set_error(GFD_EUNSUPPORTED, "direction stencil radius out of range");
+}
+
 template <class V, int MODE>
 int general_go(const gfd_operator* op, const V* in, V* out, const V* rho, int64_t nin,
                GenParams<typename vt<V>::S>& p, double* partials, cudaStream_t s) {
@@ -534,6 +655,17 @@ int launch_general_typed(const gfd_operator* op, int mode, const void* in, void*
                          const void* rho, int64_t nin, const double* phase_cd, double w,
                          double* partials, cudaStream_t s) {
   using S = typename vt<V>::S;
+  if (dirs_eligible(op, mode)) {
+    const V* a = static_cast<const V*>(in);
+    V* b = static_cast<V*>(out);
+    const V* r = static_cast<const V*>(rho);
+    if (mode == OP_APPLY)
+      return dirs_dispatch<V, MODE_APPLY>(op, mode, a, b, nullptr, nin, phase_cd, w, nullptr, s);
+    if (mode == OP_JACOBI || mode == OP_JACOBI_NEG)
+      return dirs_dispatch<V, MODE_JACOBI>(op, mode, a, b, r, nin, phase_cd, w, nullptr, s);
+    if (mode == OP_RESIDUAL)
+      return dirs_dispatch<V, MODE_RESIDUAL>(op, mode, a, b, r, nin, phase_cd, w, partials, s);
+  }
   if (op->ncoefs > kMaxCoefs) return set_error(GFD_EUNSUPPORTED, "too many stencil coefficients");
   GenParams<S> p{};
   p.n0 = op->n[0]; p.n1 = op->n[1]; p.n2 = op->n[2];
@@ -567,6 +699,10 @@ inline int64_t partials_count(const gfd_operator* op, int64_t nin) {
     LaunchGeom g = star_geom(op, tile, nin, op->R);
     int gx = (op->n[2] + td.BZ - 1) / td.BZ, gy = (op->n[1] + td.BY - 1) / td.BY;
     return (int64_t)gx * gy * g.nxc * nin;
+  }
+  if (dirs_eligible(op, OP_RESIDUAL)) {
+    const DirGeom g = dirs_geom(op, nin);
+    return (int64_t)g.gx * g.gy * g.nxc * nin;
   }
   const int BZ = 32, BY = 8;
   LaunchGeom g = star_geom(op, TILE_WIDE, nin, std::max(op->mp, 1));

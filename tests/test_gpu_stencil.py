@@ -210,6 +210,43 @@ def test_multicolour_gauss_seidel(golden, cuda, tag):
     assert rel_err(host(phi), ref) < TOL
 
 
+DIRECTION_GRIDS = [((4, 4, 4), 1), ((6, 11, 49), (1, 0, 1)), ((9, 50, 48), 1), ((17, 7, 97), 0),
+                   ((8, 130, 5), (0, 1, 1))]
+
+
+@pytest.mark.parametrize('N,pbc', DIRECTION_GRIDS)
+@pytest.mark.parametrize('R', [1, 2, 3, 4])
+def test_direction_stencils(cuda, N, pbc, R):
+    """Offsets k d over random subsets of the 13 lattice directions, weights
+    without any symmetry: tile edges (48 columns, 10 rows), single rows,
+    periodic axes as short as the reach; apply, and the Jacobi sweep."""
+    from gpaw_b200.fd_operators import FDOperator
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    gd = GridDescriptor(N, np.array(N) * 0.25, pbc)
+    rng = np.random.default_rng(10 * R + N[0])
+    dirs = np.indices((3, 3, 3)).reshape(3, -1).T[-13:] - 1
+    pick = rng.permutation(13)[:rng.integers(4, 14)]
+    offs, coefs = [(0, 0, 0)], [-9.0]
+    for d in dirs[pick]:
+        for k in range(1, R + 1):
+            for s in (1, -1):
+                offs.append(tuple(s * k * d))
+                coefs.append(rng.uniform(-1, 1) / len(pick))
+    args = (N, np.array(N) * 0.25, pbc)
+    a = rng.standard_normal((2,) + tuple(gd.n_c))
+    assert rel_err(gpu_apply(cuda, args, coefs, offs, a), K.fd_apply(coefs, offs, gd.pbc_c, a)) < TOL
+    ac = a + 1j * rng.standard_normal(a.shape)
+    ph = np.exp(2j * np.pi * gd.sdisp_cd * np.array([0.17, -0.31, 0.4])[:, None])
+    assert rel_err(gpu_apply(cuda, args, coefs, offs, ac, ph),
+                   K.fd_apply(coefs, offs, gd.pbc_c, ac, ph)) < TOL
+    phi, rho = a[0].copy(), a[1].copy()
+    op = FDOperator(coefs, offs, gd)
+    t = dev(phi, cuda)
+    op.relax(2, t, dev(rho, cuda), 2, 0.7)
+    K.relax(2, coefs, offs, gd.pbc_c, phi, rho, 2, 0.7)
+    assert rel_err(host(t), phi) < TOL
+
+
 BLOCKED_SHAPES = [((24, 16, 33), 1), ((40, 20, 36), 1), ((40, 20, 36), 0), ((17, 18, 40), (0, 1, 1)),
                   ((9, 33, 64), (1, 1, 0))]
 

@@ -177,7 +177,9 @@ TuneKey star_tune_key(const gfd_operator* op, int dtype, int mode, int64_t nin) 
   k.n0 = op->n[0];
   k.n1 = op->n[1];
   k.n2 = op->n[2];
-  k.order = op->R;
+  // Applies of one-axis stencils run other kernels than the Laplacian of the
+  // same grid and radius: a key of their own.
+  k.order = op->R + (mode == OP_APPLY ? 64 * (line_axis(op) + 1) : 0);
   k.per = per_mask(op->per);
   k.nbc = band_class(nin);
   return k;

@@ -79,6 +79,17 @@ enum {
 inline bool tile48_eligible(const gfd_operator* op) {
   return op->star && op->R >= 1 && op->R <= 4 && op->n[2] % 48 == 0;
 }
+// The only axis a star stencil reaches along, or -1.
+inline int line_axis(const gfd_operator* op) {
+  int axis = -1;
+  for (int c = 0; c < op->ncoefs; c++)
+    for (int a = 0; a < 3; a++)
+      if (op->off[3 * c + a]) {
+        if (axis >= 0 && axis != a) return -1;
+        axis = a;
+      }
+  return op->star ? axis : -1;
+}
 enum { PLAN_DIRECT = 0, PLAN_MARCH = 1 };               // one thread per point / marching
 enum { TK_STAR = 0, TK_RESTRICT = 1, TK_INTERP = 2 };
 

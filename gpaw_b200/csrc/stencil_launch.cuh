@@ -9,6 +9,7 @@
 #include "internal.h"
 #include "stencil.cuh"
 #include "stencil_dirs.cuh"
+#include "stencil_line.cuh"
 #include "stencil_split.cuh"
 #include "stencil_tma.cuh"
 #include "stencil_tmasplit.cuh"
@@ -403,6 +404,65 @@ void star_params(const gfd_operator* op, int mode, double w, const double* phase
           p.fix_yz = 1;
 }
 
+// ---------------------------------------------------------------------------
+// Stencils along one axis (stencil_line.cuh), for applies past the
+// one-thread-per-point limit.
+// ---------------------------------------------------------------------------
+template <class V, int R>
+int line_go(const gfd_operator* op, int axis, const V* in, V* out, int64_t nin,
+            LineParams<typename vt<V>::S>& p, cudaStream_t s) {
+  const int n0 = op->n[0], n1 = op->n[1], n2 = op->n[2];
+  p.n = op->n[axis];
+  p.per = op->per[axis];
+  if (axis == 2) {
+    const int gz = (n2 + 255) / 256, bz = (n2 + gz - 1) / gz, rows = 256 / bz, passes = 8;
+    p.inner = (long long)n0 * n1 * nin;
+    p.outer = 1;
+    const long long blocks = (p.inner + (long long)rows * passes - 1) / ((long long)rows * passes);
+    if (blocks > 0x7fffffffLL) return set_error(GFD_EUNSUPPORTED, "too many rows");
+    launch_k(line_row_kernel<V, R>, dim3((unsigned)blocks, gz), rows * bz, 0, s, in, out, p, bz,
+             rows, passes);
+    return check_launch("line_row_kernel");
+  }
+  p.inner = axis == 0 ? (long long)n1 * n2 : n2;
+  p.outer = axis == 0 ? nin : nin * n0;
+  // Whole lines per thread once that fills the chip a few times over; chunks
+  // of at least 4 (2R) outputs, whose 2R extra values come from L2, below.
+  const long long threads = p.inner * p.outer, want = 4LL * 2048 * num_sms();
+  const int maxc = std::max(1, p.n / (8 * R));
+  p.nch = (int)std::min<long long>(maxc, std::max<long long>(1, want / std::max(1LL, threads)));
+  p.chunk = (p.n + p.nch - 1) / p.nch;
+  p.nch = (p.n + p.chunk - 1) / p.chunk;
+  const int nt = p.inner >= 256 ? 256 : (int)((p.inner + 31) / 32 * 32);
+  const long long gx = (p.inner + nt - 1) / nt;
+  launch_k(line_march_kernel<V, R>,
+           dim3((unsigned)gx, (unsigned)p.nch, (unsigned)std::min<long long>(p.outer, 65535)), nt,
+           0, s, in, out, p);
+  return check_launch("line_march_kernel");
+}
+
+template <class V>
+int line_dispatch(const gfd_operator* op, int axis, const V* in, V* out, int64_t nin,
+                  const double* phase_cd, cudaStream_t s) {
+  using S = typename vt<V>::S;
+  LineParams<S> p{};
+  const double* w = axis == 0 ? op->cx : axis == 1 ? op->cy : op->cz;
+  for (int i = 0; i < 2 * kMaxR + 1; i++) p.w[i] = S(w[i]);
+  p.w[kMaxR] = S(op->c0);
+  for (int d = 0; d < 2; d++)
+    p.ph[d] = {S(phase_cd ? phase_cd[4 * axis + 2 * d] : 1.0),
+               S(phase_cd ? phase_cd[4 * axis + 2 * d + 1] : 0.0)};
+  switch (op->R) {
+    case 1: return line_go<V, 1>(op, axis, in, out, nin, p, s);
+    case 2: return line_go<V, 2>(op, axis, in, out, nin, p, s);
+    case 3: return line_go<V, 3>(op, axis, in, out, nin, p, s);
+    case 4: return line_go<V, 4>(op, axis, in, out, nin, p, s);
+    case 5: return line_go<V, 5>(op, axis, in, out, nin, p, s);
+    case 6: return line_go<V, 6>(op, axis, in, out, nin, p, s);
+  }
+  return set_error(GFD_EUNSUPPORTED, "star stencil radius out of range");
+}
+
 template <class V>
 int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* out, const void* rho,
                       int64_t nin, const double* phase_cd, double w, double* partials,
@@ -432,6 +492,10 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
     if (mode == OP_RESIDUAL)
       return direct_dispatch<V, MODE_RESIDUAL>(op, vin, vout, vrho, p, total, s);
     return direct_dispatch<V, MODE_APPLY>(op, vin, vout, nullptr, p, total, s);
+  }
+  if (mode == OP_APPLY) {
+    const int axis = line_axis(op);
+    if (axis >= 0) return line_dispatch<V>(op, axis, vin, vout, nin, phase_cd, s);
   }
   if constexpr (std::is_same_v<V, cplx<double>>) {
     if (!tuned && mode == OP_APPLY && tma_eligible(op, in)) {

@@ -247,6 +247,31 @@ def test_direction_stencils(cuda, N, pbc, R):
     assert rel_err(host(t), phi) < TOL
 
 
+@pytest.mark.parametrize('N,pbc', [((71, 64, 67), 1), ((3, 300, 340), 0), ((340, 3, 300), (1, 0, 1)),
+                                   ((20, 60, 270), (0, 1, 1))])
+@pytest.mark.parametrize('axis,n', [(0, 1), (0, 6), (1, 2), (1, 3), (2, 3), (2, 4)])
+def test_one_axis_stencils(cuda, N, pbc, axis, n):
+    """Central differences along one axis, with a centre weight, past the
+    one-thread-per-point size: chunked lines, rows longer than a block, axes
+    shorter than the reach (zero boundary), phases; real and complex."""
+    if np.ravel(pbc * np.ones(3, int))[axis] and N[axis] < n:
+        pytest.skip('periodic axis shorter than the stencil')
+    offs = [[0, 0, 0]]
+    for k in range(1, n + 1):
+        for s in (k, -k):
+            offs.append([s if c == axis else 0 for c in range(3)])
+    rng = np.random.default_rng(n + axis)
+    coefs = rng.uniform(-1, 1, len(offs))
+    gd = G.Grid(N, np.array(N) * 0.25, pbc)
+    args = (N, np.array(N) * 0.25, pbc)
+    a = rng.standard_normal((3,) + tuple(gd.n_c))
+    assert rel_err(gpu_apply(cuda, args, coefs, offs, a), K.fd_apply(coefs, offs, gd.pbc_c, a)) < TOL
+    ac = a + 1j * rng.standard_normal(a.shape)
+    ph = G.bloch_phases(gd, (0.17, -0.31, 0.4))
+    assert rel_err(gpu_apply(cuda, args, coefs, offs, ac, ph),
+                   K.fd_apply(coefs, offs, gd.pbc_c, ac, ph)) < TOL
+
+
 BLOCKED_SHAPES = [((24, 16, 33), 1), ((40, 20, 36), 1), ((40, 20, 36), 0), ((17, 18, 40), (0, 1, 1)),
                   ((9, 33, 64), (1, 1, 0))]
 

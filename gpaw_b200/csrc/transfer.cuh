@@ -455,13 +455,6 @@ interp_kernel(const V* __restrict__ in, V* out, const V* base,
   }
 }
 
-// ---------------------------------------------------------------------------
-// Direct forms for small grids (coarse multigrid levels): one thread per
-// output point, the three 1-D passes nested in registers in the reference's
-// order (axis 2 innermost, then axis 1, then axis 0), neighbours read through
-// the L1 cache.  The marching kernels above pay a memory round trip per plane,
-// which dominates on grids of a few thousand points.
-// ---------------------------------------------------------------------------
 // Input position u of an axis: element offset (always inside the band) in
 // units of the axis stride, whether it holds a value, and its wrap side.
 struct TrTap {
@@ -474,6 +467,112 @@ __device__ __forceinline__ TrTap tr_map(int u, int n, int per, int stride) {
   t.off = map_axis(u, n, per, t.side, t.ok) * stride;
   return t;
 }
+
+// A value where even, the K-tap value of `get` where odd; both are computed
+// for nn = 1 (a select, so no lane waits for another's path), the wider taps
+// branch.
+template <int NN, class V, class Get>
+__device__ __forceinline__ V ip_along(int odd, Get get) {
+  if constexpr (NN == 1) {
+    const V a = get(0), m = ip_tap<NN, V>([&](int o) { return o == 0 ? a : get(odd); });
+    V r;
+    if constexpr (vt<V>::NC == 2) r = {odd ? m.re : a.re, odd ? m.im : a.im};
+    else r = odd ? m : a;
+    return r;
+  } else {
+    return odd ? ip_tap<NN, V>(get) : get(0);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Two-tap restriction (nn = 1: the multigrid V-cycle, the band preconditioner)
+// on large grids.  With three taps per axis a point needs so few neighbours
+// that staging them in shared memory costs more than reading them through L1
+// (the staged kernel's two barriers per plane and its one plane of prefetch
+// kept it at a fifth of the memory rate: 493 us for 32 complex128 bands of
+// 96^3): a thread owns one output column and marches along axis 0, carrying
+// the in-plane value of the plane that two outputs share.  Per coarse plane it
+// makes the in-plane values of two fine planes from 18 independent loads (2.25
+// per fine point).  Registers are held to 6 (complex128) or 8 blocks of 128
+// threads per SM: with all 18 values in flight per thread (138 registers, one
+// block of 256) the same case took 227 us.
+// ---------------------------------------------------------------------------
+constexpr int kTwoTapNT = 128;
+template <class V>
+__global__ void __launch_bounds__(kTwoTapNT, sizeof(V) >= 16 ? 6 : 8)
+restrict1_kernel(const V* __restrict__ in, V* __restrict__ out,
+                 const TrParams<typename vt<V>::S> p) {
+  pdl_enter();
+  using S = typename vt<V>::S;
+  const int plane_out = p.no1 * p.no2, g = blockIdx.x * kTwoTapNT + threadIdx.x;
+  if (g >= plane_out) return;
+  const int Y = g / p.no2, Z = g - Y * p.no2;
+  const int bnd = blockIdx.y / p.nxc, xc = blockIdx.y % p.nxc;
+  const int X0 = xc * p.x_chunk, X1 = min(p.no0, X0 + p.x_chunk);
+  const V* inb = in + bnd * p.band_in;
+  V* outb = out + bnd * p.band_out;
+  TrTap ty[3], tz[3];
+  bool ok = true, side = false;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    ty[k] = tr_map(2 * Y + k - p.lo1, p.ni1, p.per1, p.ni2);
+    tz[k] = tr_map(2 * Z + k - p.lo2, p.ni2, p.per2, 1);
+    ok = ok && ty[k].ok && tz[k].ok;
+    side = side || ty[k].side >= 0 || tz[k].side >= 0;
+  }
+  const long long plane_in = (long long)p.ni1 * p.ni2;
+  // In-plane value of fine plane f (axis 2 innermost, as the reference).
+  auto value = [&](int f) -> V {
+    int xs;
+    const int x = wrap_plane(f, p.ni0, p.per0, xs);
+    if (x < 0) return vzero<V>();
+    const V* a = inb + x * plane_in;
+    V v[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int k = 0; k < 3; k++) v[i][k] = ldro(a + (ty[i].off + tz[k].off));
+    if (!ok) {
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) v[i][k] = value_or_zero(ty[i].ok && tz[k].ok, v[i][k]);
+    }
+    if constexpr (vt<V>::NC == 2) {
+      if (xs >= 0 || side) {
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+          for (int k = 0; k < 3; k++) {
+            if (xs >= 0) v[i][k] = phase_mul(phase_of(p.P, 0, xs), v[i][k]);
+            v[i][k] = side_phase(p.P, 1, ty[i].side, v[i][k]);
+            v[i][k] = side_phase(p.P, 2, tz[k].side, v[i][k]);
+          }
+      }
+    }
+    return rst_tap<1, V>([&](int oy) {
+      return rst_tap<1, V>([&](int oz) { return v[oy + 1][oz + 1]; });
+    });
+  };
+  V prev = value(2 * X0 - p.lo0);
+  for (int X = X0; X < X1; X++) {
+    const V c = value(2 * X + 1 - p.lo0), next = value(2 * X + 2 - p.lo0);
+    V v = rst_tap<1, V>([&](int o) { return o == 0 ? c : (o < 0 ? prev : next); });
+    prev = next;
+    if (p.out_scale != S(1)) v = vmul(p.out_scale, v);
+    const long long o = (long long)X * plane_out + g;
+    stcs(outb + o, v);
+    if (p.seed) stcs(static_cast<V*>(p.seed) + bnd * p.band_out + o, vmul(p.seed_scale, v));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Direct forms for small grids (coarse multigrid levels): one thread per
+// output point, the three 1-D passes nested in registers in the reference's
+// order (axis 2 innermost, then axis 1, then axis 0), neighbours read through
+// the L1 cache.  The marching kernels above pay a memory round trip per plane,
+// which dominates on grids of a few thousand points.
+// ---------------------------------------------------------------------------
 template <class LD, class V, class S>
 __device__ __forceinline__ V tr_fetch(const V* base, const TrTap& x, const TrTap& y,
                                       const TrTap& z, const TrParams<S>& p) {
@@ -540,22 +639,6 @@ __device__ __forceinline__ V restrict_point(const V* __restrict__ in,
   const int r1 = int(rem - X * plane_out);
   const int Y = r1 / p.no2, Z = r1 - Y * p.no2;
   return restrict_point_at<V, NN, LD>(in + b * p.band_in, X, Y, Z, p);
-}
-
-// A value where even, the K-tap value of `get` where odd; both are computed
-// for nn = 1 (a select, so no lane waits for another's path), the wider taps
-// branch.
-template <int NN, class V, class Get>
-__device__ __forceinline__ V ip_along(int odd, Get get) {
-  if constexpr (NN == 1) {
-    const V a = get(0), m = ip_tap<NN, V>([&](int o) { return o == 0 ? a : get(odd); });
-    V r;
-    if constexpr (vt<V>::NC == 2) r = {odd ? m.re : a.re, odd ? m.im : a.im};
-    else r = odd ? m : a;
-    return r;
-  } else {
-    return odd ? ip_tap<NN, V>(get) : get(0);
-  }
 }
 
 // One interpolated point at output coordinates (X, Y, Z), times out_scale

@@ -69,6 +69,30 @@ int interp_go(const gfd_transformer* tr, const V* in, V* out, const V* base, int
   return check_launch("interp_kernel");
 }
 
+// Two-tap restriction past the one-thread-per-point limit: output planes in
+// blocks of 128 columns, axis 0 cut into chunks of at least 4 output planes
+// until about 16 blocks per SM are in flight.
+template <class V>
+int restrict1_go(const gfd_transformer* tr, const V* in, V* out, int64_t nin,
+                 TrParams<typename vt<V>::S>& p, int cps, cudaStream_t s) {
+  const int gx = (tr->nout[1] * tr->nout[2] + kTwoTapNT - 1) / kTwoTapNT;
+  const int64_t tiles = (int64_t)gx * nin;
+  const int64_t target = 4LL * (cps > 0 ? cps : march_ctas_per_sm()) * num_sms();
+  const int maxc = std::max(1, tr->nout[0] / 4);
+  const int nxc = (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles));
+  p.x_chunk = (tr->nout[0] + nxc - 1) / nxc;
+  p.nxc = (tr->nout[0] + p.x_chunk - 1) / p.x_chunk;
+  const int64_t per_launch = std::max<int64_t>(1, 65535 / p.nxc);
+  V* seed = static_cast<V*>(p.seed);
+  for (int64_t b0 = 0; b0 < nin; b0 += per_launch) {
+    const int64_t nb = std::min<int64_t>(per_launch, nin - b0);
+    p.seed = seed ? seed + b0 * p.band_out : nullptr;
+    launch_k(restrict1_kernel<V>, dim3(gx, (unsigned)(nb * p.nxc)), kTwoTapNT, 0, s,
+             in + b0 * p.band_in, out + b0 * p.band_out, p);
+  }
+  return check_launch("restrict1_kernel");
+}
+
 // Outputs (all bands) up to direct_max_points() use the one-thread-per-point
 // forms.
 template <class V, int NN>
@@ -120,7 +144,7 @@ int tr_typed(const gfd_transformer* tr, const void* in, void* out, const void* b
   } else {
     if (base) return set_error(GFD_EINVAL, "subtracting form is for interpolation only");
     switch (tr->nn) {
-      case 1: return restrict_go<V, 1>(tr, vin, vout, nin, p, cps, s);
+      case 1: return restrict1_go<V>(tr, vin, vout, nin, p, cps, s);
       case 2: return restrict_go<V, 2>(tr, vin, vout, nin, p, cps, s);
       case 3: return restrict_go<V, 3>(tr, vin, vout, nin, p, cps, s);
       case 4: return restrict_go<V, 4>(tr, vin, vout, nin, p, cps, s);

@@ -74,6 +74,23 @@ def test_transform_shapes(cuda, N, pbc, nn):
         assert rel_err(o32.astype(float), ref) < 2e-6
 
 
+@pytest.mark.parametrize('N,pbc,nb', [((66, 90, 110), 1, 4), ((66, 90, 110), 0, 4),
+                                      ((4, 34, 38), (1, 0, 1), 1100), ((150, 22, 18), (0, 1, 0), 50)])
+def test_two_tap_marching(cuda, N, pbc, nb):
+    """nn = 1 past the one-thread-per-point size: chunked axis 0, partial
+    column blocks, many short bands; real and phased complex."""
+    og = G.Grid(N, np.array(N) * 0.3, pbc)
+    gd = product_grid(og)
+    rng = np.random.default_rng(nb)
+    for g2, o2, nin in ((gd.coarsen(), og.coarsen(), 8 * nb), (gd.refine(), og.refine(), nb)):
+        a = rng.uniform(-1, 1, (nin,) + tuple(og.n_c))
+        assert rel_err(gpu_transform(cuda, gd, g2, 1, a), K.transform(og, o2, 1, a, nthreads=8)) < TOL
+        ac = a[:nb] + 1j * a[-nb:]
+        ph = G.bloch_phases(og, (0.25, -0.125, 0.3))
+        assert rel_err(gpu_transform(cuda, gd, g2, 1, ac, ph),
+                       K.transform(og, o2, 1, ac, ph, nthreads=8)) < TOL
+
+
 def test_transformations_conserve_integral(cuda):
     """gpaw/test/transformations.py:9-48 on the GPU."""
     from gpaw_b200.grid_descriptor import GridDescriptor

@@ -415,13 +415,16 @@ int line_go(const gfd_operator* op, int axis, const V* in, V* out, int64_t nin,
   p.n = op->n[axis];
   p.per = op->per[axis];
   if (axis == 2) {
-    const int gz = (n2 + 255) / 256, bz = (n2 + gz - 1) / gz, rows = 256 / bz, passes = 8;
+    const int rows = std::max(1, 256 / n2);
     p.inner = (long long)n0 * n1 * nin;
     p.outer = 1;
+    // up to 40 KB of staged rows, so several blocks share an SM
+    const size_t row_b = size_t(rows) * (n2 + 2 * R) * sizeof(V);
+    const int passes = (int)std::max<size_t>(1, std::min<size_t>(kLinePasses, 40 * 1024 / row_b));
     const long long blocks = (p.inner + (long long)rows * passes - 1) / ((long long)rows * passes);
     if (blocks > 0x7fffffffLL) return set_error(GFD_EUNSUPPORTED, "too many rows");
-    launch_k(line_row_kernel<V, R>, dim3((unsigned)blocks, gz), rows * bz, 0, s, in, out, p, bz,
-             rows, passes);
+    launch_k(line_row_kernel<V, R>, dim3((unsigned)blocks), rows * n2, passes * row_b, s, in, out,
+             p, rows, passes);
     return check_launch("line_row_kernel");
   }
   p.inner = axis == 0 ? (long long)n1 * n2 : n2;
@@ -495,7 +498,8 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
   }
   if (mode == OP_APPLY) {
     const int axis = line_axis(op);
-    if (axis >= 0) return line_dispatch<V>(op, axis, vin, vout, nin, phase_cd, s);
+    if (axis >= 0 && (axis < 2 || op->n[2] <= 1024))
+      return line_dispatch<V>(op, axis, vin, vout, nin, phase_cd, s);
   }
   if constexpr (std::is_same_v<V, cplx<double>>) {
     if (!tuned && mode == OP_APPLY && tma_eligible(op, in)) {

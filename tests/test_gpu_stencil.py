@@ -210,6 +210,29 @@ def test_multicolour_gauss_seidel(golden, cuda, tag):
     assert rel_err(host(phi), ref) < TOL
 
 
+@pytest.mark.parametrize('where', [(3, 5, 7), (0, 0, 0), (19, 59, 46)])
+@pytest.mark.parametrize('value', [float('inf'), float('nan')])
+def test_non_finite_values_stay_within_reach(cuda, where, value):
+    """An infinity or NaN reaches the outputs whose stencil holds it and no
+    others, whatever the tile."""
+    import torch
+    from gpaw_b200.fd_operators import Gradient, Laplace
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    N = (20, 60, 47)
+    gd = GridDescriptor(N, np.array(N) * 0.25, 1)
+    for dtype in (float, complex):
+        for op in (Laplace(gd, -0.5, 3, dtype), Gradient(gd, 2, 1.0, 3, dtype)):
+            a = torch.zeros((8,) + N, dtype=op.dtype, device=cuda)
+            a[5][where] = value
+            out = torch.empty_like(a)
+            op.apply(a, out, None if dtype is float else np.ones((3, 2), complex))
+            bad = ~torch.isfinite(torch.view_as_real(out).sum(-1) if dtype is complex else out)
+            want = torch.zeros_like(bad)
+            for off in op.offset_pc:
+                want[(5,) + tuple((w - int(d)) % m for w, d, m in zip(where, off, N))] = True
+            assert torch.equal(bad, want)
+
+
 DIRECTION_GRIDS = [((4, 4, 4), 1), ((6, 11, 49), (1, 0, 1)), ((9, 50, 48), 1), ((17, 7, 97), 0),
                    ((8, 130, 5), (0, 1, 1))]
 

@@ -56,7 +56,8 @@ class TunePlan(ctypes.Structure):
 
     def as_dict(self):
         return {'form': ('direct', 'march')[self.form],
-                'tile': (32, 16, 8, '32x8', 'split', 'tma-split', '48x8')[self.tile],
+                'tile': (32, 16, 8, '32x8', 'split', 'tma-split', '48x8', 'pair',
+                         '48x16', 'flex')[self.tile],
                 'ctas_per_sm': self.ctas_per_sm, 'us': self.us}
 
 # Every function the header declares: name -> (restype, argtypes).

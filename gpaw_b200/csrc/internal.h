@@ -67,6 +67,8 @@ int num_sms();
 // 48 columns by 8 rows (48 x 4 threads, 2 rows each, two CTAs per SM), for
 // axis-2 lengths that are multiples of 48: it stages 2R halo columns per 48
 // where the 32-column tiles stage 2R per 32.
+// TILE_48R: real bands, radius <= 3, 48 columns by 16 rows (48 x 4 threads, 4
+// rows each), where 48-column tiles pad axis 2 less than 32-column ones.
 enum {
   TILE_WIDE = 0,
   TILE_MID = 1,
@@ -74,10 +76,14 @@ enum {
   TILE_SHORT = 3,
   TILE_SPLIT = 4,
   TILE_TMASPLIT = 5,
-  TILE_48 = 6
+  TILE_48 = 6,
+  TILE_48R = 8
 };
 inline bool tile48_eligible(const gfd_operator* op) {
   return op->star && op->R >= 1 && op->R <= 4 && op->n[2] % 48 == 0;
+}
+inline bool tile48r_eligible(const gfd_operator* op) {
+  return op->star && op->R == 3 && op->n[2] > 32 && (op->n[2] + 47) / 48 * 48 < (op->n[2] + 31) / 32 * 32;
 }
 // The only axis a star stencil reaches along, or -1.
 inline int line_axis(const gfd_operator* op) {

@@ -378,7 +378,9 @@ typedef struct gfd_tune_plan {
                        4 complex bands with re / im on lane pairs (radius <= 3),
                        5 the same for complex128 on full rows staged by TMA,
                        6 complex128, 48 columns x 8 rows (axis-2 lengths that are
-                       multiples of 48) */
+                       multiples of 48), 7 complex128 apply of radius 3, two
+                       columns per lane pair, 8 real bands, 48 columns x 16 rows,
+                       9 complex128 up to radius 3, tile sides that fit the grid */
   int ctas_per_sm;  /* axis-0 split target */
   double us;        /* measured time per launch, microseconds */
 } gfd_tune_plan;

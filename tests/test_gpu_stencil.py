@@ -210,6 +210,40 @@ def test_multicolour_gauss_seidel(golden, cuda, tag):
     assert rel_err(host(phi), ref) < TOL
 
 
+TILE_GRIDS = [((10, 24, 32), 1), ((7, 96, 32), 0), ((6, 12, 96), (1, 0, 1)), ((9, 90, 100), 1),
+              ((8, 33, 65), (0, 1, 0)), ((40, 3, 129), 1), ((6, 131, 7), (1, 0, 1)),
+              ((11, 47, 47), 0)]
+
+
+@pytest.mark.parametrize('N,pbc', TILE_GRIDS)
+@pytest.mark.parametrize('n', [1, 2, 3])
+def test_fitted_tiles(cuda, N, pbc, n):
+    """Band batches past the one-thread-per-point size on grids around the
+    fitted tiles' edges (32, 48 and 64 columns, rows in twos and threes, one
+    row or column over): apply and apply with a potential, real and phased
+    complex128, and the Jacobi sweep of one large grid."""
+    import torch
+    from gpaw_b200.fd_operators import FDOperator
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    gd = GridDescriptor(N, np.array(N) * 0.25, pbc)
+    c, o = G.laplace_stencil(G.Grid(N, np.array(N) * 0.25, pbc), -0.5, n)
+    nb = 300000 // int(np.prod(gd.n_c)) + 2
+    rng = np.random.default_rng(n)
+    v = rng.standard_normal(tuple(gd.n_c))
+    a = rng.standard_normal((nb,) + tuple(gd.n_c))
+    ph = np.exp(2j * np.pi * gd.sdisp_cd * np.array([0.17, -0.31, 0.4])[:, None])
+    for x, p in ((a, None), (a + 1j * a[::-1], ph)):
+        t = dev(x, cuda)
+        op = FDOperator(c, o, gd, t.dtype)
+        ref = K.fd_apply(c, o, gd.pbc_c, x, p, nthreads=8)
+        out = torch.full_like(t, float('nan'))
+        op.apply(t, out, p)
+        assert rel_err(host(out), ref) < TOL
+        out.fill_(float('nan'))
+        op.apply_with_potential(t, out, dev(v, cuda), p)
+        assert rel_err(host(out), ref + v * x) < TOL
+
+
 @pytest.mark.parametrize('where', [(3, 5, 7), (0, 0, 0), (19, 59, 46)])
 @pytest.mark.parametrize('value', [float('inf'), float('nan')])
 def test_non_finite_values_stay_within_reach(cuda, where, value):

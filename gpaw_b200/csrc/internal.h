@@ -67,6 +67,10 @@ int num_sms();
 // 48 columns by 8 rows (48 x 4 threads, 2 rows each, two CTAs per SM), for
 // axis-2 lengths that are multiples of 48: it stages 2R halo columns per 48
 // where the 32-column tiles stage 2R per 32.
+// TILE_PAIR: complex128 apply of radius 3, star_pair_kernel (two columns by
+// three rows per lane pair, 32 columns by 12 rows).
+// TILE_FLEX: complex128, radius <= 3, star_flex_kernel (tile sides that fit the
+// grid).
 // TILE_48R: real bands, radius <= 3, 48 columns by 16 rows (48 x 4 threads, 4
 // rows each), where 48-column tiles pad axis 2 less than 32-column ones.
 enum {
@@ -77,7 +81,9 @@ enum {
   TILE_SPLIT = 4,
   TILE_TMASPLIT = 5,
   TILE_48 = 6,
-  TILE_48R = 8
+  TILE_PAIR = 7,
+  TILE_48R = 8,
+  TILE_FLEX = 9
 };
 inline bool tile48_eligible(const gfd_operator* op) {
   return op->star && op->R >= 1 && op->R <= 4 && op->n[2] % 48 == 0;

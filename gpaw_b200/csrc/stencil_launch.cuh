@@ -9,7 +9,9 @@
 #include "internal.h"
 #include "stencil.cuh"
 #include "stencil_dirs.cuh"
+#include "stencil_flex.cuh"
 #include "stencil_line.cuh"
+#include "stencil_pair.cuh"
 #include "stencil_split.cuh"
 #include "stencil_tma.cuh"
 #include "stencil_tmasplit.cuh"
@@ -410,6 +412,139 @@ void star_params(const gfd_operator* op, int mode, double w, const double* phase
 }
 
 // ---------------------------------------------------------------------------
+// complex128 bands up to radius 3: star_flex_kernel and star_pair_kernel.
+// ---------------------------------------------------------------------------
+// Axis-0 chunks and launches of a tiling with gx x gy tiles per plane.
+template <class F>
+int march_launches(const gfd_operator* op, int gx, int gy, int64_t nin, int cps,
+                   StarParams<double>& p, F launch) {
+  const int64_t tiles = (int64_t)gx * gy * nin;
+  const int64_t target = (int64_t)(cps > 0 ? cps : march_ctas_per_sm()) * num_sms();
+  const int maxc = std::max(1, op->n[0] / std::max(4, 2 * op->R));
+  const int nxc = (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles));
+  p.x_chunk = (op->n[0] + nxc - 1) / nxc;
+  p.nxc = (op->n[0] + p.x_chunk - 1) / p.x_chunk;
+  const int64_t per_launch = std::max<int64_t>(1, 65535 / p.nxc);
+  for (int64_t b0 = 0; b0 < nin; b0 += per_launch) {
+    const int64_t nb = std::min<int64_t>(per_launch, nin - b0);
+    launch(dim3(gx, gy, (unsigned)(nb * p.nxc)), b0 * p.band);
+  }
+  return GFD_OK;
+}
+
+// The tile with the least work per plane, threads that run plus a quarter per
+// staged cell; a narrower tile has to save 6% (its rows start more staged
+// segments).  Measured for 108^3 R = 3: (36, 6) 692 us, (36, 7) 725, (54, 4)
+// 796; 90 x 100: (50, 5) 430, (26, 9) and (34, 7) slower; 96^2: (32, 8) 928,
+// (48, 5) 989, (48, 4) 1006.
+inline FlexTile flex_tile(const gfd_operator* op, int mode) {
+  const int n1 = op->n[1], n2 = op->n[2], R = op->R;
+  // two CTAs per SM
+  const size_t most_smem = 112 * 1024 - (mode == OP_APPLY ? 0 : mode == OP_POTENTIAL ? 16 : 32) * 1024;
+  FlexTile best = {std::min(n2, 8), 1};
+  double cost = 0.0;
+  int last = 0;
+  for (int gx = (n2 + kFlexBZ - 1) / kFlexBZ; gx <= n2; gx++) {
+    FlexTile t;
+    t.bz = (n2 + gx - 1) / gx;
+    if (t.bz == last) continue;
+    last = t.bz;
+    if (t.bz < 16 && cost > 0.0) break;
+    double c_bz = 0.0;
+    int ty_bz = 1;
+    const int most = std::min(kFlexNT / t.bz, (n1 + kFlexVY - 1) / kFlexVY);
+    for (t.ty = 1; t.ty <= most; t.ty++) {
+      if (flex_cells(t, R) > kFlexCPT * kFlexNT ||
+          size_t(kFlexStages) * (t.ty * kFlexVY + 2 * R) * (kFlexBZ + 2 * R) * 16 > most_smem)
+        break;
+      const double tiles = double((n2 + t.bz - 1) / t.bz) *
+                           ((n1 + t.ty * kFlexVY - 1) / (t.ty * kFlexVY));
+      const double c = tiles * (t.bz * t.ty + 0.25 * flex_cells(t, R));
+      if (c_bz == 0.0 || c < c_bz) {
+        c_bz = c;
+        ty_bz = t.ty;
+      }
+    }
+    if (c_bz > 0.0 && (cost == 0.0 || c_bz < 0.94 * cost)) {
+      cost = c_bz;
+      best = {t.bz, ty_bz};
+    }
+  }
+  return best;
+}
+// Points of the padded plane of a tile.
+inline long long padded(int n1, int n2, int by, int bz) {
+  return (long long)((n1 + by - 1) / by * by) * ((n2 + bz - 1) / bz * bz);
+}
+// Built-in choice for complex128 up to radius 3 past the one-thread-per-point
+// size (`fixed`: the fixed-side tile that would be taken).  Applies: the pair
+// kernel at radius 3 where its 32 x 12 tiles pad either axis by 3% at most
+// (4424 against 3949 GB/s on 96^3, 4169 against 3908 on 128 x 120 x 128, but 3733
+// against 3983 on 64^3), else the flex kernel (64^3 3983 against 3691 for the
+// 32 x 8 tile, 90 x 100 3598 against 2867; radius 1 5998 against 5248, radius
+// 2 4287 against 4010).  The other modes: flex where the fixed tile pads the
+// plane 8% more (potential 90 x 100: 3237 against 2521, but 3113 against 3639
+// on 96^2 for the 48 x 8 tile; Jacobi 104^2 2623 against 1929, but 2619
+// against 2685 on 96^2).
+inline int c128_tile(const gfd_operator* op, int mode, int fixed) {
+  const int n1 = op->n[1], n2 = op->n[2];
+  if (mode == OP_APPLY && op->R == kPairR) {
+    const int gx = (n2 + kPairBZ - 1) / kPairBZ, by = 4 * kPairVY, gy = (n1 + by - 1) / by;
+    if (gx * kPairBZ - n2 <= n2 / 32 && gy * by - n1 <= n1 / 32) return TILE_PAIR;
+  }
+  if (mode == OP_APPLY) return TILE_FLEX;
+  const FlexTile f = flex_tile(op, mode);
+  const TileDims td = tile_dims(fixed);
+  return padded(n1, n2, td.BY, td.BZ) * 100 > padded(n1, n2, f.ty * kFlexVY, f.bz) * 108
+             ? TILE_FLEX
+             : fixed;
+}
+
+inline int pair_launch(const gfd_operator* op, const cplx<double>* in, cplx<double>* out,
+                       int64_t nin, StarParams<double> p, int cps, cudaStream_t s) {
+  // 32 columns by 12 rows; fewer where the grid is smaller
+  const int gx = (op->n[2] + kPairBZ - 1) / kPairBZ;
+  PairTile t;
+  t.bz = ((op->n[2] + gx - 1) / gx + 1) / 2 * 2;
+  t.ty = std::min(4, (op->n[1] + kPairVY - 1) / kPairVY);
+  const int gy = (op->n[1] + t.ty * kPairVY - 1) / (t.ty * kPairVY);
+  const size_t smem = pair_smem_bytes(t.ty);
+  int st = raise_smem_limit(star_pair_kernel, smem, "cudaFuncSetAttribute(star_pair_kernel)");
+  if (st) return st;
+  march_launches(op, gx, gy, nin, cps, p, [&](dim3 grid, long long off) {
+    launch_k(star_pair_kernel, grid, kPairNT, smem, s, in + off, out + off, p, t);
+  });
+  return check_launch("star_pair_kernel");
+}
+
+template <int R, int MODE>
+int flex_go(const gfd_operator* op, int mode, const cplx<double>* in, cplx<double>* out,
+            const cplx<double>* rho, int64_t nin, StarParams<double> p, int cps, cudaStream_t s) {
+  const FlexTile t = flex_tile(op, mode);
+  const int gx = (op->n[2] + t.bz - 1) / t.bz;
+  const int gy = (op->n[1] + t.ty * kFlexVY - 1) / (t.ty * kFlexVY);
+  auto kern = star_flex_kernel<R, MODE>;
+  const size_t smem = flex_smem_bytes<R, MODE>(t);
+  int st = raise_smem_limit(kern, smem, "cudaFuncSetAttribute(star_flex_kernel)");
+  if (st) return st;
+  march_launches(op, gx, gy, nin, cps, p, [&](dim3 grid, long long off) {
+    launch_k(kern, grid, kFlexNT, smem, s, in + off, out + off, rho ? rho + off : nullptr, p, t);
+  });
+  return check_launch("star_flex_kernel");
+}
+template <int MODE>
+int flex_dispatch(const gfd_operator* op, int mode, const cplx<double>* in, cplx<double>* out,
+                  const cplx<double>* rho, int64_t nin, const StarParams<double>& p, int cps,
+                  cudaStream_t s) {
+  switch (op->R) {
+    case 1: return flex_go<1, MODE>(op, mode, in, out, rho, nin, p, cps, s);
+    case 2: return flex_go<2, MODE>(op, mode, in, out, rho, nin, p, cps, s);
+    case 3: return flex_go<3, MODE>(op, mode, in, out, rho, nin, p, cps, s);
+  }
+  return set_error(GFD_EUNSUPPORTED, "flex stencil: radius <= 3");
+}
+
+// ---------------------------------------------------------------------------
 // Stencils along one axis (stencil_line.cuh), for applies past the
 // one-thread-per-point limit.
 // ---------------------------------------------------------------------------
@@ -530,11 +665,19 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
   // complex64 (512-band 96^3 Laplace): 2970-2990 GB/s against 2905-2918 for
   // the 32 x 16 tile
   if (t48ok && !shortok && tile == TILE_WIDE) tile = TILE_48;
+  const bool flexok = sizeof(V) >= 16 && op->R <= kFlexR;
+  const bool pairok = sizeof(V) >= 16 && op->R == kPairR && mode == OP_APPLY;
+  if (flexok && (tile == TILE_WIDE || tile == TILE_SHORT || tile == TILE_48))
+    tile = c128_tile(op, mode, tile);
   // real bands: 16 of 47^3 17.7 us against 21.1 us (two 32-column tiles)
   const bool t48rok = vt<V>::NC == 1 && mode != OP_RESIDUAL && tile48r_eligible(op);
   if (t48rok && tile == TILE_WIDE) tile = TILE_48R;
   if (tuned) {
-    if (plan.tile == TILE_48R)
+    if (plan.tile == TILE_PAIR)
+      tile = pairok ? TILE_PAIR : tile;
+    else if (plan.tile == TILE_FLEX)
+      tile = flexok ? TILE_FLEX : tile;
+    else if (plan.tile == TILE_48R)
       tile = t48rok ? TILE_48R : tile;
     else if (plan.tile == TILE_SHORT)
       tile = shortok ? TILE_SHORT : tile;
@@ -557,6 +700,19 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
       if (mode == OP_RESIDUAL)
         return ts_dispatch(op, MODE_RESIDUAL, vin, vout, vrho, nullptr, nin, p, cps, s);
       return ts_dispatch(op, MODE_APPLY, vin, vout, nullptr, nullptr, nin, p, cps, s);
+    }
+  }
+  if constexpr (std::is_same_v<V, cplx<double>>) {
+    const int cps = tuned ? plan.cps : 0;
+    if (tile == TILE_PAIR) return pair_launch(op, vin, vout, nin, p, cps, s);
+    if (tile == TILE_FLEX) {
+      if (mode == OP_POTENTIAL)
+        return flex_dispatch<MODE_POTENTIAL>(op, mode, vin, vout, nullptr, nin, p, cps, s);
+      if (mode == OP_JACOBI || mode == OP_JACOBI_NEG)
+        return flex_dispatch<MODE_JACOBI>(op, mode, vin, vout, vrho, nin, p, cps, s);
+      if (mode == OP_RESIDUAL)
+        return flex_dispatch<MODE_RESIDUAL>(op, mode, vin, vout, vrho, nin, p, cps, s);
+      return flex_dispatch<MODE_APPLY>(op, mode, vin, vout, nullptr, nin, p, cps, s);
     }
   }
   LaunchGeom g = star_geom(op, tile, nin, op->R, tuned ? plan.cps : 0);

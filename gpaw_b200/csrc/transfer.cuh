@@ -180,7 +180,6 @@ restrict_kernel(const V* __restrict__ in, V* __restrict__ out,
   constexpr int RZ = 2 * BZC - 1 + 2 * W;
   constexpr int CELLS = RY * RZ;
   constexpr int CC = (CELLS + NT - 1) / NT;
-  constexpr int QL = 2 * W + 1;           // fine planes feeding one coarse plane
   // Each staged fine row holds its even positions first, then its odd ones:
   // the axis-2 taps of neighbouring coarse points are then consecutive
   // words (a stride-2 read would hit every bank twice).
@@ -238,14 +237,10 @@ restrict_kernel(const V* __restrict__ in, V* __restrict__ out,
     }
   };
 
-  V q[VYC][QL];
-#pragma unroll
-  for (int j = 0; j < VYC; j++)
-#pragma unroll
-    for (int k = 0; k < QL; k++) q[j][k] = vzero<V>();
-
   load(fbeg);
-  for (int f = fbeg; f < fend; ++f) {
+  // The in-plane values of fine plane f at this thread's coarse points: stage
+  // the plane, axis-2 pass, axis-1 pass.
+  auto in_plane = [&](int f, V (&v)[VYC]) {
     V* Fb = F + (f & 1) * STG;
     V* Tb = T + (f & 1) * RY * BZC;
 #pragma unroll
@@ -280,33 +275,64 @@ restrict_kernel(const V* __restrict__ in, V* __restrict__ out,
       }
     }
     __syncthreads();
-    // axis-1 pass for this thread's coarse points, pushed into the queue
+    if constexpr (VYC == 2) {
+      // axis-1 pass, adjacent coarse rows 2 ty and 2 ty + 1: as for the column
+      // pairs, 2nn + 3 reads instead of 2 (2nn + 1)
+      const V* col = Tb + 4 * ty * BZC + tz;
+      V tap[2 * NN + 1];
+#pragma unroll
+      for (int m = 0; m <= 2 * NN; m++) tap[m] = col[2 * m * BZC];
+      const V c0 = col[W * BZC], c1 = col[(W + 2) * BZC];
+      v[0] = rst_tap<NN, V>([&](int o) { return o == 0 ? c0 : tap[(o + W) >> 1]; });
+      v[1] = rst_tap<NN, V>([&](int o) { return o == 0 ? c1 : tap[((o + W) >> 1) + 1]; });
+    } else {
+      static_assert(VYC == 1, "one or two coarse rows per thread");
+      const V* col = Tb + (2 * ty + W) * BZC + tz;
+      v[0] = rst_tap<NN, V>([&](int o) { return col[o * BZC]; });
+    }
+  };
+
+  // axis-0 pass: fine planes 2h and 2h + 1 past fbeg.  The first is an odd
+  // neighbour of coarse planes X0 + h - m, m = 0 .. W, whose sums stay in
+  // registers (s[.][m]); the second is the centre of X0 + h - (nn - 1).
+  V s[VYC][W + 1];
+#pragma unroll
+  for (int j = 0; j < VYC; j++)
+#pragma unroll
+    for (int m = 0; m <= W; m++) s[j][m] = vzero<V>();
+  const int last = X1 - X0 + W - 1;
+  for (int h = 0; h <= last; h++) {
+    V v[VYC];
+    in_plane(fbeg + 2 * h, v);
 #pragma unroll
     for (int j = 0; j < VYC; j++) {
-      const V* col = Tb + (2 * (ty + j * TYC) + W) * BZC + tz;
-      V v = rst_tap<NN, V>([&](int o) { return col[o * BZC]; });
 #pragma unroll
-      for (int k = 0; k + 1 < QL; k++) q[j][k] = q[j][k + 1];
-      q[j][QL - 1] = v;
+      for (int m = W; m > 0; m--) s[j][m] = s[j][m - 1];
+      s[j][0] = vzero<V>();
+#pragma unroll
+      for (int m = 0; m <= W; m++) {
+        const int d = 2 * m - W, k = ((d < 0 ? -d : d) - 1) / 2;
+        madd(s[j][m], lagw<NN, S>(k), v[j]);
+      }
     }
-    // axis-0 pass: the queue centre is fine plane f - W
-    const int fc = f - W;
-    const int rel = fc - W + p.lo0;
-    if (f - fbeg >= QL - 1 && (rel & 1) == 0) {
-      const int X = rel >> 1;
-      if (X >= X0 && X < X1) {
+    const int X = X0 + h - W;
+    if (X >= X0) {
 #pragma unroll
-        for (int j = 0; j < VYC; j++) {
-          const int y = Y0 + ty + j * TYC, z = Z0 + tz;
-          if (y < p.no1 && z < p.no2) {
-            V v = rst_tap<NN, V>([&](int o) { return q[j][W + o]; });
-            if (p.out_scale != S(1)) v = vmul(p.out_scale, v);
-            const long long o = X * plane_out + (long long)y * p.no2 + z;
-            stcs(outb + o, v);
-            if (p.seed) stcs(static_cast<V*>(p.seed) + (outb - out) + o, vmul(p.seed_scale, v));
-          }
+      for (int j = 0; j < VYC; j++) {
+        const int y = Y0 + ty * VYC + j, z = Z0 + tz;
+        if (y < p.no1 && z < p.no2) {
+          V r = vmul(S(0.5), s[j][W]);
+          if (p.out_scale != S(1)) r = vmul(p.out_scale, r);
+          const long long o = X * plane_out + (long long)y * p.no2 + z;
+          stcs(outb + o, r);
+          if (p.seed) stcs(static_cast<V*>(p.seed) + (outb - out) + o, vmul(p.seed_scale, r));
         }
       }
+    }
+    if (h < last) {
+      in_plane(fbeg + 2 * h + 1, v);
+#pragma unroll
+      for (int j = 0; j < VYC; j++) s[j][NN - 1] = vadd(s[j][NN - 1], v[j]);
     }
   }
 }

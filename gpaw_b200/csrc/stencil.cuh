@@ -741,4 +741,61 @@ color_gs_star_kernel(V* phi, const V* __restrict__ rho, const V* frozen,
   }
 }
 
+// Gauss-Seidel sweeps on a colour-split copy.  A colour's points lie R + 1
+// apart in a row, so the lanes of color_gs_star_kernel read one value out of
+// each 32-byte sector, 8 shared-memory-rate cycles per load at R = 3.  In the
+// copy each row holds its points of equal i2 mod NC together (NC = R + 1 runs
+// that fill the row exactly): a point's neighbours are then consecutive words
+// across lanes for all 6R taps.  Zero boundaries only (a periodic sweep needs
+// the scratch grid for its starting values).
+template <int NC>
+__device__ __forceinline__ int gs_run(int phase, int n2) {  // start of a run
+  const int q = n2 / NC, rem = n2 - q * NC;
+  return phase * q + min(phase, rem);
+}
+// to != 0: copy = split(phi); else phi = joined(copy).
+template <class V, int NC>
+__global__ void __launch_bounds__(256)
+gs_split_kernel(V* __restrict__ phi, V* __restrict__ copy, int n2, int n, int to) {
+  pdl_enter();
+  for (int g = blockIdx.x * 256 + threadIdx.x; g < n; g += gridDim.x * 256) {
+    const int row = g / n2, z = g - row * n2;
+    const int c = row * n2 + gs_run<NC>(z % NC, n2) + z / NC;
+    if (to) copy[c] = phi[g];
+    else phi[g] = copy[c];
+  }
+}
+template <class V, int R>
+__global__ void __launch_bounds__(256)
+color_gs_split_kernel(V* phi, const V* __restrict__ rho, const StarParams<typename vt<V>::S> p,
+                      int color) {
+  pdl_enter();
+  using S = typename vt<V>::S;
+  constexpr int NC = R + 1;
+  const int slots = gs_row_slots(p.n2, NC), pl = p.n1 * p.n2;
+  const int nq = p.n0 * p.n1 * slots;
+  for (int q = blockIdx.x * 256 + threadIdx.x; q < nq; q += gridDim.x * 256) {
+    int i0, i1, i2;
+    if (!gs_colour_point(q, slots, NC, color, p.n1, p.n2, i0, i1, i2)) continue;
+    const int first = i2 % NC, j = i2 / NC;
+    const int rowb = (i0 * p.n1 + i1) * p.n2, at = rowb + gs_run<NC>(first, p.n2) + j;
+    S sx = 0, sy = 0, sz = 0;  // summed as in gs_star_point_at
+#pragma unroll
+    for (int k = -R; k <= R; k++) {
+      if (k == 0) continue;
+      const bool xok = unsigned(i0 + k) < unsigned(p.n0), yok = unsigned(i1 + k) < unsigned(p.n1);
+      const bool zok = unsigned(i2 + k) < unsigned(p.n2);
+      const V vx = value_or_zero(xok, phi[xok ? at + k * pl : at]);
+      const V vy = value_or_zero(yok, phi[yok ? at + k * p.n2 : at]);
+      const int tz = first + k + NC;  // >= 1
+      const int zat = rowb + gs_run<NC>(tz % NC, p.n2) + j + tz / NC - 1;
+      const V vz = value_or_zero(zok, phi[zok ? zat : at]);
+      madd(sx, p.cx[kMaxR + k], vx);
+      madd(sy, p.cy[kMaxR + k], vy);
+      madd(sz, p.cz[kMaxR + k], vz);
+    }
+    phi[at] = (rho[rowb + i2] - (sx + (sy + sz))) * p.wc;
+  }
+}
+
 }  // namespace gfd

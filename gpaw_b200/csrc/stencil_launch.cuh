@@ -989,6 +989,24 @@ int gs_sweeps(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* froz
   return check_launch("color_gs_kernel");
 }
 
+// The same on a colour-split copy in the scratch grid, from kGsSplitPoints
+// points of a zero-boundary grid up.
+constexpr long long kGsSplitPoints = 40000;
+template <class V, int R>
+int gs_split_sweeps(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* copy,
+                    const StarParams<typename vt<V>::S>& p, cudaStream_t s) {
+  const int n = (int)p.band, NC = R + 1;
+  const int nq = p.n0 * p.n1 * gs_row_slots(p.n2, NC);
+  const int cap = 148 * 16;
+  const int nb = std::min((n + 255) / 256, cap), qb = std::min((nq + 255) / 256, cap);
+  launch_k(gs_split_kernel<V, R + 1>, nb, 256, 0, s, phi, copy, p.n2, n, 1);
+  for (int sw = 0; sw < nsweeps; sw++)
+    for (int c = 0; c < NC; c++)
+      launch_k(color_gs_split_kernel<V, R>, qb, 256, 0, s, copy, rho, p, c);
+  launch_k(gs_split_kernel<V, R + 1>, nb, 256, 0, s, phi, copy, p.n2, n, 0);
+  return check_launch("color_gs_split_kernel");
+}
+
 template <class V>
 int gs_typed(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* frozen, int ncolor,
              cudaStream_t s) {
@@ -996,6 +1014,11 @@ int gs_typed(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* froze
   if (op->star) {
     StarParams<S> p;
     gs_star_params(op, p);
+    if (!op->per[0] && !op->per[1] && !op->per[2] && p.band >= kGsSplitPoints && nsweeps > 0 &&
+        ncolor == op->R + 1) {
+      if (op->R == 2) return gs_split_sweeps<V, 2>(op, phi, rho, nsweeps, frozen, p, s);
+      if (op->R == 3) return gs_split_sweeps<V, 3>(op, phi, rho, nsweeps, frozen, p, s);
+    }
     switch (op->R) {
       case 1: return gs_sweeps<V, 1>(op, phi, rho, nsweeps, frozen, ncolor, p, s);
       case 2: return gs_sweeps<V, 2>(op, phi, rho, nsweeps, frozen, ncolor, p, s);

@@ -210,6 +210,23 @@ def test_multicolour_gauss_seidel(golden, cuda, tag):
     assert rel_err(host(phi), ref) < TOL
 
 
+@pytest.mark.parametrize('N,nn', [((37, 41, 34), 3), ((36, 40, 43), 3), ((44, 36, 33), 2),
+                                  ((35, 36, 37), 2)])
+def test_colour_split_gauss_seidel(cuda, N, nn):
+    """Zero-boundary grids past the size from which Gauss-Seidel works on a
+    colour-split copy, every remainder of the row length by the colour count:
+    two sweeps against the colour-by-colour reference."""
+    from gpaw_b200.fd_operators import FDOperator
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    gd = GridDescriptor(N, tuple(0.3 * x for x in N), False)
+    c, o = G.laplace_stencil(G.Grid(N, tuple(0.3 * x for x in N), False), -0.25 / np.pi, nn)
+    rng = np.random.RandomState(4)
+    phi0, rho = (rng.standard_normal(tuple(gd.n_c)) for _ in range(2))
+    phi = dev(phi0, cuda)
+    FDOperator(c, o, gd, float).relax(1, phi, dev(rho, cuda), 2)
+    assert rel_err(host(phi), multicolour_gs_reference(c, o, gd.pbc_c, phi0, rho, 2)) < TOL
+
+
 TILE_GRIDS = [((10, 24, 32), 1), ((7, 96, 32), 0), ((6, 12, 96), (1, 0, 1)), ((9, 90, 100), 1),
               ((8, 33, 65), (0, 1, 0)), ((40, 3, 129), 1), ((6, 131, 7), (1, 0, 1)),
               ((11, 47, 47), 0)]

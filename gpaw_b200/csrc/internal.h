@@ -154,10 +154,12 @@ int tr_launch_seed(const gfd_transformer* tr, int dtype, const void* in, void* o
                    double seed_scale, cudaStream_t s);
 // General form: out = out_scale * transfer(in) (interpolation with base:
 // out = base - out_scale * interpolate(in)); restriction with seed also
-// writes seed = seed_scale * out.  out_scale must be 1 or -1 (exact).
+// writes seed = seed_scale * out.  out_scale must be 1 or -1 (exact);
+// interpolation with total (a device scalar): the factor target / *total.
 int tr_launch_ex(const gfd_transformer* tr, int dtype, const void* in, void* out,
                  const void* base, int64_t nin, const double* phases, double out_scale,
-                 void* seed, double seed_scale, cudaStream_t s);
+                 void* seed, double seed_scale, cudaStream_t s, const double* total = nullptr,
+                 double target = 0.0);
 // Interpolation with the correction fused: out = base - interpolate(in)
 // (in place when base == out).
 int tr_launch_sub(const gfd_transformer* tr, int dtype, const void* in, void* out,

@@ -199,7 +199,7 @@ g_tr_kernel(const GTr* __restrict__ items, int nitems, int ntiles, unsigned* ctr
       const int r1 = g - X * plane;
       const int Y = r1 / sp.no2, Z = r1 - Y * sp.no2;
       if constexpr (INTERP) {
-        it.out[g] = interp_point_at<double, NN, true, LoadRO>(it.in, it.base + g, X, Y, Z, sp);
+        it.out[g] = interp_point_at<double, NN, true, LoadRO>(it.in, it.base + g, X, Y, Z, sp, sp.out_scale);
       } else {
         const double v = restrict_point_at<double, NN, LoadRO>(it.in, X, Y, Z, sp);
         it.out[g] = v;

@@ -75,7 +75,15 @@ struct TrParams {
   // Factor on the transferred value (1, or -1 for the negated transfers of
   // the band preconditioner; multiplying by -1 is exact).
   S out_scale;
+  // Interpolation only: when total != nullptr the factor is target / *total
+  // instead (a device scalar that an earlier kernel on the stream wrote).
+  const double* total;
+  double target;
 };
+template <class S>
+__device__ __forceinline__ S out_factor(const TrParams<S>& p) {
+  return p.total ? S(p.target / *p.total) : p.out_scale;
+}
 
 // Transfer parameters of a transformer (host side).
 template <class S>
@@ -366,6 +374,7 @@ interp_kernel(const V* __restrict__ in, V* out, const V* base,
   const int X0 = xc * p.x_chunk, X1 = min(p.no0, X0 + p.x_chunk);
   const long long plane_in = (long long)p.ni1 * p.ni2;
   const long long plane_out = (long long)p.no1 * p.no2;
+  const S osc = out_factor(p);
   const V* inb = in + bnd * p.band_in;
   V* outb = out + bnd * p.band_out;
   const V* baseb = SUB ? base + bnd * p.band_out : nullptr;
@@ -471,7 +480,7 @@ interp_kernel(const V* __restrict__ in, V* out, const V* base,
           if (y < p.no1 && z < p.no2) {
             V v = par ? ip_tap<NN, V>([&](int o) { return q[j][NN - 1 + o]; }) : q[j][NN - 1];
             const long long o = X * plane_out + (long long)y * p.no2 + z;
-            if (p.out_scale != S(1)) v = vmul(p.out_scale, v);
+            if (osc != S(1)) v = vmul(osc, v);
             if constexpr (SUB) v = vsub(baseb[o], v);
             stcs(outb + o, v);
           }
@@ -667,12 +676,13 @@ __device__ __forceinline__ V restrict_point(const V* __restrict__ in,
   return restrict_point_at<V, NN, LD>(in + b * p.band_in, X, Y, Z, p);
 }
 
-// One interpolated point at output coordinates (X, Y, Z), times out_scale
+// One interpolated point at output coordinates (X, Y, Z), times osc
 // (SUB: *bo, the base value at that point, minus it).  For nn = 1 the eight
 // corner loads are independent (an even axis reads its one point twice).
 template <class V, int NN, bool SUB, class LD>
 __device__ __forceinline__ V interp_point_at(const V* __restrict__ base, const V* bo, int X, int Y,
-                                             int Z, const TrParams<typename vt<V>::S>& p) {
+                                             int Z, const TrParams<typename vt<V>::S>& p,
+                                             typename vt<V>::S osc) {
   // g = f + skip[c][0]; even g: coarse point c(i) = i + nn - 1 - lo, odd: between c(i), c(i)+1
   const int gx = X + p.sk0, gy = Y + p.sk1, gz = Z + p.sk2;
   const int cx = (gx >> 1) + NN - 1 - p.lo0, cy = (gy >> 1) + NN - 1 - p.lo1,
@@ -689,7 +699,7 @@ __device__ __forceinline__ V interp_point_at(const V* __restrict__ base, const V
       });
     });
   });
-  if (p.out_scale != typename vt<V>::S(1)) v = vmul(p.out_scale, v);
+  if (osc != typename vt<V>::S(1)) v = vmul(osc, v);
   if constexpr (SUB) v = vsub(b, v);
   return v;
 }
@@ -697,7 +707,8 @@ __device__ __forceinline__ V interp_point_at(const V* __restrict__ base, const V
 // The same at flat index g over all output bands.
 template <class V, int NN, bool SUB, class LD>
 __device__ __forceinline__ V interp_point(const V* __restrict__ in, const V* base_out,
-                                          const TrParams<typename vt<V>::S>& p, long long g) {
+                                          const TrParams<typename vt<V>::S>& p,
+                                          typename vt<V>::S osc, long long g) {
   const long long plane_out = (long long)p.no1 * p.no2;
   const long long b = g / p.band_out;
   const long long rem = g - b * p.band_out;
@@ -705,7 +716,7 @@ __device__ __forceinline__ V interp_point(const V* __restrict__ in, const V* bas
   const int r1 = int(rem - X * plane_out);
   const int Y = r1 / p.no2, Z = r1 - Y * p.no2;
   return interp_point_at<V, NN, SUB, LD>(in + b * p.band_in, SUB ? base_out + g : nullptr, X, Y,
-                                         Z, p);
+                                         Z, p, osc);
 }
 
 template <class V, int NN>
@@ -725,8 +736,9 @@ __global__ void __launch_bounds__(256)
 interp_direct_kernel(const V* __restrict__ in, V* out, const V* base_out,
                      const TrParams<typename vt<V>::S> p, long long total) {
   pdl_enter();
+  const auto osc = out_factor(p);
   for (long long g = blockIdx.x * 256LL + threadIdx.x; g < total; g += (long long)gridDim.x * 256)
-    out[g] = interp_point<V, NN, SUB, LoadRO>(in, base_out, p, g);
+    out[g] = interp_point<V, NN, SUB, LoadRO>(in, base_out, p, osc, g);
 }
 
 }  // namespace gfd

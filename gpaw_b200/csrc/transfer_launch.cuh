@@ -113,10 +113,12 @@ int direct_go(const gfd_transformer* tr, const V* in, V* out, const V* base, int
 template <class V>
 int tr_typed(const gfd_transformer* tr, const void* in, void* out, const void* base_v,
              int64_t nin, const double* ph, cudaStream_t s, void* seed, double seed_scale,
-             double out_scale) {
+             double out_scale, const double* total, double target) {
   using S = typename vt<V>::S;
   TrParams<S> p;
   tr_params(tr, ph, seed, seed_scale, out_scale, p);
+  p.total = total;
+  p.target = target;
   if (seed && tr->interpolate) return set_error(GFD_EINVAL, "seeded form is for restriction only");
   const V* vin = static_cast<const V*>(in);
   V* vout = static_cast<V*>(out);
@@ -159,5 +161,6 @@ int tr_typed(const gfd_transformer* tr, const void* in, void* out, const void* b
 #define GFD_DECLARE_TRANSFER_ENTRY(NAME)                                                      \
   namespace gfd {                                                                             \
   int transfer_##NAME(const gfd_transformer*, const void*, void*, const void*, int64_t,       \
-                      const double*, cudaStream_t, void*, double, double);                    \
+                      const double*, cudaStream_t, void*, double, double, const double*,      \
+                      double);                                                                \
   }

@@ -16,17 +16,22 @@ namespace gfd {
 
 int tr_launch_ex(const gfd_transformer* tr, int dtype, const void* in, void* out,
                  const void* base, int64_t nin, const double* phases, double out_scale,
-                 void* seed, double seed_scale, cudaStream_t s) {
+                 void* seed, double seed_scale, cudaStream_t s, const double* total,
+                 double target) {
   if (nin <= 0) return GFD_OK;
   switch (dtype) {
     case GFD_FLOAT64:
-      return transfer_f64(tr, in, out, base, nin, phases, s, seed, seed_scale, out_scale);
+      return transfer_f64(tr, in, out, base, nin, phases, s, seed, seed_scale, out_scale, total,
+                          target);
     case GFD_FLOAT32:
-      return transfer_f32(tr, in, out, base, nin, phases, s, seed, seed_scale, out_scale);
+      return transfer_f32(tr, in, out, base, nin, phases, s, seed, seed_scale, out_scale, total,
+                          target);
     case GFD_COMPLEX128:
-      return transfer_c128(tr, in, out, base, nin, phases, s, seed, seed_scale, out_scale);
+      return transfer_c128(tr, in, out, base, nin, phases, s, seed, seed_scale, out_scale, total,
+                          target);
     case GFD_COMPLEX64:
-      return transfer_c64(tr, in, out, base, nin, phases, s, seed, seed_scale, out_scale);
+      return transfer_c64(tr, in, out, base, nin, phases, s, seed, seed_scale, out_scale, total,
+                          target);
   }
   return set_error(GFD_EINVAL, "unknown dtype");
 }

@@ -70,16 +70,49 @@ __global__ void __launch_bounds__(256) add_potential_kernel(V* __restrict__ out,
   }
 }
 
-// y[i] *= target / *total (total on the device, computed by an earlier
-// kernel on the stream).
-static __global__ void __launch_bounds__(256) scale_to_total_kernel(double* __restrict__ y, long long n,
-                                                             double target,
-                                                             const double* __restrict__ total) {
+// Per-block partial sums, in a fixed order, of the fine-grid sum of an
+// interpolation, from the coarse values alone: a coarse point's weight is the
+// product over the axes of the interpolation weights it has in all fine
+// points (2 per axis away from zero boundaries).  An eighth of the data of a
+// sum over the result, which then need not be read and scaled afterwards.
+struct InterpSum {
+  int n[3], nf[3], per[3];  // coarse and fine points, boundary
+  int shift[3];             // fine index of coarse point c is 2 c + shift
+  int nn;
+  double w[4];              // Lagrange weights by distance
+};
+__device__ __forceinline__ double interp_weight(const InterpSum& p, int a, int c) {
+  const int nn = p.nn, f = 2 * c + p.shift[a], nf = p.nf[a];
+  if (p.per[a] || (f - 2 * nn + 1 >= 0 && f + 2 * nn - 1 < nf)) return 2.0;
+  double s = f >= 0 && f < nf ? 1.0 : 0.0;
+  for (int k = 0; k < nn; k++) {
+    const int hi = f + 2 * k + 1, lo = f - 2 * k - 1;
+    if (hi >= 0 && hi < nf) s += p.w[k];
+    if (lo >= 0 && lo < nf) s += p.w[k];
+  }
+  return s;
+}
+static __global__ void __launch_bounds__(kRedThreads) interp_sum_kernel(
+    const double* __restrict__ a, long long total, const InterpSum p,
+    double* __restrict__ partials) {
   pdl_enter();
-  const double x = target / *total;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    y[i] *= x;
+  __shared__ double red[kRedThreads / 32];
+  const int band = p.n[0] * p.n[1] * p.n[2];
+  double s = 0.0;
+  for (long long i = blockIdx.x * (long long)kRedThreads + threadIdx.x; i < total;
+       i += (long long)gridDim.x * kRedThreads) {
+    const int g = int(i % band), row = g / p.n[2], z = g - row * p.n[2];
+    const int x = row / p.n[1], y = row - x * p.n[1];
+    s += a[i] * (interp_weight(p, 0, x) * interp_weight(p, 1, y) * interp_weight(p, 2, z));
+  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double b = 0.0;
+    for (int w = 0; w < kRedThreads / 32; w++) b += red[w];
+    partials[blockIdx.x] = b;
+  }
 }
 
 // Per-block partial sums of a[i] (SQUARE: a[i]^2), in a fixed order.

@@ -467,49 +467,60 @@ __device__ __forceinline__ V star_point_at(const V* __restrict__ base, const V* 
   V s = vmul(cc, LD::ld(base + rem));
   // 32-bit offsets: a band holds fewer than 2^27 points.
   const int pl = p.n1 * p.n2, row = i0 * pl + i1 * p.n2, ownr = int(rem);
+  V src = vzero<V>();
+  if constexpr (MODE == MODE_JACOBI || MODE == MODE_RESIDUAL) src = LD::ld(rho_b + rem);
+  // All loads first: left to itself the compiler keeps to 32 registers and
+  // waits for one neighbour after the other.
+  V v[3][2 * R];
 #pragma unroll
-  for (int k = -R; k <= R; k++) {
-    if (k == 0) continue;
+  for (int k = 0; k < 2 * R; k++) {
+    const int d = k < R ? k - R : k - R + 1;
     int sd;
     bool ok;
-    int j = map_axis(i0 + k, p.n0, p.per0, sd, ok);
-    V v = value_or_zero(ok, LD::ld(base + (j * pl + (ownr - i0 * pl))));
-    madd(s, p.cx[kMaxR + k], side_phase(p.P, 0, sd, v));
-    j = map_axis(i1 + k, p.n1, p.per1, sd, ok);
-    v = value_or_zero(ok, LD::ld(base + (i0 * pl + j * p.n2 + i2)));
-    madd(s, p.cy[kMaxR + k], side_phase(p.P, 1, sd, v));
-    j = map_axis(i2 + k, p.n2, p.per2, sd, ok);
-    v = value_or_zero(ok, LD::ld(base + (row + j)));
-    madd(s, p.cz[kMaxR + k], side_phase(p.P, 2, sd, v));
+    int j = map_axis(i0 + d, p.n0, p.per0, sd, ok);
+    v[0][k] = side_phase(p.P, 0, sd, value_or_zero(ok, LD::ld(base + (j * pl + (ownr - i0 * pl)))));
+    j = map_axis(i1 + d, p.n1, p.per1, sd, ok);
+    v[1][k] = side_phase(p.P, 1, sd, value_or_zero(ok, LD::ld(base + (i0 * pl + j * p.n2 + i2))));
+    j = map_axis(i2 + d, p.n2, p.per2, sd, ok);
+    v[2][k] = side_phase(p.P, 2, sd, value_or_zero(ok, LD::ld(base + (row + j))));
   }
-  if constexpr (MODE == MODE_JACOBI) return vmul(p.wc, vsub(LD::ld(rho_b + rem), s));
-  else if constexpr (MODE == MODE_RESIDUAL) return vsub(s, LD::ld(rho_b + rem));
+#pragma unroll
+  for (int k = 0; k < 2 * R; k++) {
+    const int d = k < R ? k - R : k - R + 1;
+    madd(s, p.cx[kMaxR + d], v[0][k]);
+    madd(s, p.cy[kMaxR + d], v[1][k]);
+    madd(s, p.cz[kMaxR + d], v[2][k]);
+  }
+  if constexpr (MODE == MODE_JACOBI) return vmul(p.wc, vsub(src, s));
+  else if constexpr (MODE == MODE_RESIDUAL) return vsub(s, src);
   else return s;
 }
 
-// The same at flat index g over all bands.
+// The same at flat index g over all bands.  32-bit arithmetic (the launch
+// keeps the points of one launch below 2^31): the two 64-bit divisions it took
+// before were most of a thread's 261 instructions at R = 1.
 template <class V, int R, int MODE, class LD>
 __device__ __forceinline__ V star_point(const V* __restrict__ in, const V* __restrict__ rho,
-                                        const StarParams<typename vt<V>::S>& p, long long g) {
-  const long long plane = (long long)p.n1 * p.n2;
-  const long long b = g / p.band;
-  const long long rem = g - b * p.band;
-  const int i0 = int(rem / plane);
-  const int r1 = int(rem - i0 * plane);
-  const int i1 = r1 / p.n2, i2 = r1 - i1 * p.n2;
-  return star_point_at<V, R, MODE, LD>(in + b * p.band, rho ? rho + b * p.band : nullptr, p, i0,
-                                       i1, i2, rem);
+                                        const StarParams<typename vt<V>::S>& p, int g,
+                                        int total) {
+  const int band = int(p.band);
+  const int b = total == band ? 0 : g / band;
+  const int rem = g - b * band;
+  const int row = rem / p.n2, i2 = rem - row * p.n2;
+  const int i0 = row / p.n1, i1 = row - i0 * p.n1;
+  const long long off = (long long)b * band;
+  return star_point_at<V, R, MODE, LD>(in + off, rho ? rho + off : nullptr, p, i0, i1, i2, rem);
 }
 
 template <class V, int R, int MODE>
 __global__ void __launch_bounds__(256)
 star_direct_kernel(const V* __restrict__ in, V* __restrict__ out, const V* __restrict__ rho,
-                   const StarParams<typename vt<V>::S> p, long long total) {
+                   const StarParams<typename vt<V>::S> p, int total) {
   pdl_enter();
   __shared__ double red[8];
   double sumsq = 0.0;
-  for (long long g = blockIdx.x * 256LL + threadIdx.x; g < total; g += (long long)gridDim.x * 256) {
-    const V o = star_point<V, R, MODE, LoadRO>(in, rho, p, g);
+  for (long long g = blockIdx.x * 256 + threadIdx.x; g < total; g += gridDim.x * 256) {
+    const V o = star_point<V, R, MODE, LoadRO>(in, rho, p, int(g), total);
     out[g] = o;
     if constexpr (MODE == MODE_RESIDUAL && vt<V>::NC == 1) sumsq += sq(o);
   }
@@ -664,6 +675,20 @@ __device__ __forceinline__ void gs_point_at(V* phi, const V* __restrict__ rho, c
   phi[g] = (rho[g] - s) * (S(1) / p.coefs[0]);
 }
 
+// New value from the neighbours' values v[axis][k] (offsets -R .. -1, 1 .. R).
+template <class V, int R>
+__device__ __forceinline__ V gs_update(const V (&v)[3][2 * R], V src,
+                                       const StarParams<typename vt<V>::S>& p) {
+  typename vt<V>::S s[3] = {0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < 2 * R; k++) {
+    const int d = k < R ? k - R : k - R + 1;
+    madd(s[0], p.cx[kMaxR + d], v[0][k]);
+    madd(s[1], p.cy[kMaxR + d], v[1][k]);
+    madd(s[2], p.cz[kMaxR + d], v[2][k]);
+  }
+  return (src - (s[0] + (s[1] + s[2]))) * p.wc;
+}
 // The same for an axis-aligned stencil of radius R (p.c0 the diagonal, p.wc
 // its reciprocal).  Every neighbour's load is independent, so the update
 // costs about one memory round trip; the loop over an offset table above
@@ -675,23 +700,21 @@ __device__ __forceinline__ void gs_star_point_at(V* phi, const V* __restrict__ r
   using S = typename vt<V>::S;
   static_assert(vt<V>::NC == 1, "Gauss-Seidel works on real arrays");
   const int pl = p.n1 * p.n2, row = i0 * pl + i1 * p.n2, g = row + i2;
-  S sx = 0, sy = 0, sz = 0;
+  const V src = rho[g];
+  V v[3][2 * R];  // all loads first, as in star_point_at
 #pragma unroll
-  for (int k = -R; k <= R; k++) {
-    if (k == 0) continue;
+  for (int k = 0; k < 2 * R; k++) {
+    const int d = k < R ? k - R : k - R + 1;
     int sd;
     bool ok;
-    int j = map_axis(i0 + k, p.n0, p.per0, sd, ok);
-    const V vx = value_or_zero(ok, (sd >= 0 ? frozen : phi)[j * pl + (g - i0 * pl)]);
-    j = map_axis(i1 + k, p.n1, p.per1, sd, ok);
-    const V vy = value_or_zero(ok, (sd >= 0 ? frozen : phi)[i0 * pl + j * p.n2 + i2]);
-    j = map_axis(i2 + k, p.n2, p.per2, sd, ok);
-    const V vz = value_or_zero(ok, (sd >= 0 ? frozen : phi)[row + j]);
-    madd(sx, p.cx[kMaxR + k], vx);
-    madd(sy, p.cy[kMaxR + k], vy);
-    madd(sz, p.cz[kMaxR + k], vz);
+    int j = map_axis(i0 + d, p.n0, p.per0, sd, ok);
+    v[0][k] = value_or_zero(ok, (sd >= 0 ? frozen : phi)[j * pl + (g - i0 * pl)]);
+    j = map_axis(i1 + d, p.n1, p.per1, sd, ok);
+    v[1][k] = value_or_zero(ok, (sd >= 0 ? frozen : phi)[i0 * pl + j * p.n2 + i2]);
+    j = map_axis(i2 + d, p.n2, p.per2, sd, ok);
+    v[2][k] = value_or_zero(ok, (sd >= 0 ? frozen : phi)[row + j]);
   }
-  phi[g] = (rho[g] - (sx + (sy + sz))) * p.wc;
+  phi[g] = gs_update<V, R>(v, src, p);
 }
 
 // Points of one colour, enumerated without idle threads: index q covers

@@ -66,14 +66,39 @@ int raise_smem_limit(F* kern, size_t bytes, const char* what) {
                     what);
 }
 
+// Axis-0 chunks of a marching launch of `tiles` columns of n0 planes when
+// `resident` CTAs run at a time: the count with the fewest plane steps, a chunk
+// of c planes taking c steps, about 0.7 for each of the 2R planes around it and 3
+// to start, times the waves (at least one).  7 float64 bands of 93 x 113 x 121
+// (196 tiles): 3 chunks, 588 CTAs of 592, 44 us; 4 chunks, the former target of 4
+// CTAs per SM, 50 us.
+inline int best_chunks(int n0, int R, int64_t tiles, int64_t resident) {
+  const int most = std::max(1, n0 / std::max(4, 2 * R));
+  int best = 1;
+  double cost = 0.0;
+  for (int c = 1; c <= most; c++) {
+    const int planes = (n0 + c - 1) / c;
+    const int n = (n0 + planes - 1) / planes;
+    const double waves = std::max(1.0, double(tiles * n) / double(resident));
+    const double t = waves * (planes + 1.4 * R + 3.0);
+    if (cost == 0.0 || t < 0.98 * cost) {
+      cost = t;
+      best = n;
+    }
+  }
+  return best;
+}
+
 struct LaunchGeom {
   dim3 grid;
   int nxc, x_chunk;
   int64_t bands_per_launch;
 };
 
-inline LaunchGeom star_geom(const gfd_operator* op, int tile, int64_t nin, int R,
-                            int cps = 0) {
+// resident: CTAs per SM of the kernel where known (0: aim for march_ctas_per_sm()
+// without counting waves); cps: a launch plan's target.
+inline LaunchGeom star_geom(const gfd_operator* op, int tile, int64_t nin, int R, int cps = 0,
+                            int resident = 0) {
   TileDims td = tile_dims(tile);
   LaunchGeom g;
   int gx = (op->n[2] + td.BZ - 1) / td.BZ;
@@ -82,11 +107,20 @@ inline LaunchGeom star_geom(const gfd_operator* op, int tile, int64_t nin, int R
   int64_t target = (int64_t)(cps > 0 ? cps : march_ctas_per_sm()) * num_sms();
   int maxc = std::max(1, op->n[0] / std::max(4, 2 * R));
   int nxc = (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles));
+  if (cps == 0 && resident > 0)
+    nxc = best_chunks(op->n[0], R, tiles, (int64_t)resident * num_sms());
   g.x_chunk = (op->n[0] + nxc - 1) / nxc;
   g.nxc = (op->n[0] + g.x_chunk - 1) / g.x_chunk;
   g.bands_per_launch = std::max<int64_t>(1, 65535 / g.nxc);
   g.grid = dim3(gx, gy, 1);
   return g;
+}
+
+// CTAs per SM of star_kernel's real tiles that are sized for it
+// (star_min_ctas), 0 for the others.
+inline int real_resident(const gfd_operator* op, int tile) {
+  if (op->R > 3) return 0;
+  return tile == TILE_WIDE ? 4 : tile == TILE_48R ? 3 : 0;
 }
 
 template <class S>
@@ -356,29 +390,38 @@ inline int star_tma_dispatch(const gfd_operator* op, const cplx<double>* in, cpl
   return set_error(GFD_EUNSUPPORTED, "TMA stencil radius out of range");
 }
 
-template <class V, int MODE>
-int direct_dispatch(const gfd_operator* op, const V* in, V* out, const V* rho,
-                    const StarParams<typename vt<V>::S>& p, long long total, cudaStream_t s) {
-  const int blocks = direct_blocks(total);
-  if constexpr (vt<V>::NC == 2 && MODE != MODE_APPLY && MODE != MODE_POTENTIAL) {
-    switch (op->R) {
-      case 1: launch_k(star_direct_kernel<V, 1, MODE>, blocks, 256, 0, s, in, out, rho, p, total); break;
-      case 2: launch_k(star_direct_kernel<V, 2, MODE>, blocks, 256, 0, s, in, out, rho, p, total); break;
-      case 3: launch_k(star_direct_kernel<V, 3, MODE>, blocks, 256, 0, s, in, out, rho, p, total); break;
-      default: return set_error(GFD_EUNSUPPORTED, "complex Jacobi/residual sweeps need radius <= 3");
-    }
-    return check_launch("star_direct_kernel");
-  }
-  switch (op->R) {
-    case 1: launch_k(star_direct_kernel<V, 1, MODE>, blocks, 256, 0, s, in, out, rho, p, total); break;
-    case 2: launch_k(star_direct_kernel<V, 2, MODE>, blocks, 256, 0, s, in, out, rho, p, total); break;
-    case 3: launch_k(star_direct_kernel<V, 3, MODE>, blocks, 256, 0, s, in, out, rho, p, total); break;
-    case 4: launch_k(star_direct_kernel<V, 4, MODE>, blocks, 256, 0, s, in, out, rho, p, total); break;
-    case 5: launch_k(star_direct_kernel<V, 5, MODE>, blocks, 256, 0, s, in, out, rho, p, total); break;
-    case 6: launch_k(star_direct_kernel<V, 6, MODE>, blocks, 256, 0, s, in, out, rho, p, total); break;
-    default: return set_error(GFD_EUNSUPPORTED, "star stencil radius out of range");
+template <class V, int R, int MODE>
+int direct_go(const gfd_operator* op, const V* in, V* out, const V* rho,
+              const StarParams<typename vt<V>::S>& p, int64_t nin, cudaStream_t s) {
+  // fewer than 2^31 points per launch
+  const int64_t most = std::max<int64_t>(1, 2000000000LL / p.band);
+  for (int64_t b0 = 0; b0 < nin; b0 += most) {
+    const int total = int(std::min<int64_t>(most, nin - b0) * p.band);
+    launch_k(star_direct_kernel<V, R, MODE>, direct_blocks(total), 256, 0, s, in + b0 * p.band,
+             out + b0 * p.band, rho ? rho + b0 * p.band : nullptr, p, total);
   }
   return check_launch("star_direct_kernel");
+}
+
+template <class V, int MODE>
+int direct_dispatch(const gfd_operator* op, const V* in, V* out, const V* rho,
+                    const StarParams<typename vt<V>::S>& p, int64_t nin, cudaStream_t s) {
+  constexpr bool RELAX = MODE != MODE_APPLY && MODE != MODE_POTENTIAL;
+  switch (op->R) {
+    case 1: return direct_go<V, 1, MODE>(op, in, out, rho, p, nin, s);
+    case 2: return direct_go<V, 2, MODE>(op, in, out, rho, p, nin, s);
+    case 3: return direct_go<V, 3, MODE>(op, in, out, rho, p, nin, s);
+  }
+  if constexpr (vt<V>::NC == 2 && RELAX) {
+    return set_error(GFD_EUNSUPPORTED, "complex Jacobi/residual sweeps need radius <= 3");
+  } else {
+    switch (op->R) {
+      case 4: return direct_go<V, 4, MODE>(op, in, out, rho, p, nin, s);
+      case 5: return direct_go<V, 5, MODE>(op, in, out, rho, p, nin, s);
+      case 6: return direct_go<V, 6, MODE>(op, in, out, rho, p, nin, s);
+    }
+    return set_error(GFD_EUNSUPPORTED, "star stencil radius out of range");
+  }
 }
 
 // Stencil parameters of a star operator for one mode (weights in the
@@ -416,12 +459,14 @@ void star_params(const gfd_operator* op, int mode, double w, const double* phase
 // ---------------------------------------------------------------------------
 // Axis-0 chunks and launches of a tiling with gx x gy tiles per plane.
 template <class F>
-int march_launches(const gfd_operator* op, int gx, int gy, int64_t nin, int cps,
+int march_launches(const gfd_operator* op, int gx, int gy, int64_t nin, int cps, int resident,
                    StarParams<double>& p, F launch) {
   const int64_t tiles = (int64_t)gx * gy * nin;
-  const int64_t target = (int64_t)(cps > 0 ? cps : march_ctas_per_sm()) * num_sms();
   const int maxc = std::max(1, op->n[0] / std::max(4, 2 * op->R));
-  const int nxc = (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles));
+  const int64_t target = (int64_t)cps * num_sms();  // a launch plan's
+  const int nxc =
+      cps > 0 ? (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles))
+              : best_chunks(op->n[0], op->R, tiles, (int64_t)resident * num_sms());
   p.x_chunk = (op->n[0] + nxc - 1) / nxc;
   p.nxc = (op->n[0] + p.x_chunk - 1) / p.x_chunk;
   const int64_t per_launch = std::max<int64_t>(1, 65535 / p.nxc);
@@ -511,7 +556,7 @@ inline int pair_launch(const gfd_operator* op, const cplx<double>* in, cplx<doub
   const size_t smem = pair_smem_bytes(t.ty);
   int st = raise_smem_limit(star_pair_kernel, smem, "cudaFuncSetAttribute(star_pair_kernel)");
   if (st) return st;
-  march_launches(op, gx, gy, nin, cps, p, [&](dim3 grid, long long off) {
+  march_launches(op, gx, gy, nin, cps, 3, p, [&](dim3 grid, long long off) {
     launch_k(star_pair_kernel, grid, kPairNT, smem, s, in + off, out + off, p, t);
   });
   return check_launch("star_pair_kernel");
@@ -527,7 +572,7 @@ int flex_go(const gfd_operator* op, int mode, const cplx<double>* in, cplx<doubl
   const size_t smem = flex_smem_bytes<R, MODE>(t);
   int st = raise_smem_limit(kern, smem, "cudaFuncSetAttribute(star_flex_kernel)");
   if (st) return st;
-  march_launches(op, gx, gy, nin, cps, p, [&](dim3 grid, long long off) {
+  march_launches(op, gx, gy, nin, cps, 2, p, [&](dim3 grid, long long off) {
     launch_k(kern, grid, kFlexNT, smem, s, in + off, out + off, rho ? rho + off : nullptr, p, t);
   });
   return check_launch("star_flex_kernel");
@@ -627,14 +672,13 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
       mode != OP_RESIDUAL && tune_lookup(star_tune_key(op, dtype_of<V>(), mode, nin), &plan);
   if (tuned ? plan.path == PLAN_DIRECT : use_direct(op, nin)) {
     p.partials = partials;
-    const long long total = (long long)p.band * nin;
     if (mode == OP_POTENTIAL)
-      return direct_dispatch<V, MODE_POTENTIAL>(op, vin, vout, nullptr, p, total, s);
+      return direct_dispatch<V, MODE_POTENTIAL>(op, vin, vout, nullptr, p, nin, s);
     if (mode == OP_JACOBI || mode == OP_JACOBI_NEG)
-      return direct_dispatch<V, MODE_JACOBI>(op, vin, vout, vrho, p, total, s);
+      return direct_dispatch<V, MODE_JACOBI>(op, vin, vout, vrho, p, nin, s);
     if (mode == OP_RESIDUAL)
-      return direct_dispatch<V, MODE_RESIDUAL>(op, vin, vout, vrho, p, total, s);
-    return direct_dispatch<V, MODE_APPLY>(op, vin, vout, nullptr, p, total, s);
+      return direct_dispatch<V, MODE_RESIDUAL>(op, vin, vout, vrho, p, nin, s);
+    return direct_dispatch<V, MODE_APPLY>(op, vin, vout, nullptr, p, nin, s);
   }
   if (mode == OP_APPLY) {
     const int axis = line_axis(op);
@@ -715,7 +759,8 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
       return flex_dispatch<MODE_APPLY>(op, mode, vin, vout, nullptr, nin, p, cps, s);
     }
   }
-  LaunchGeom g = star_geom(op, tile, nin, op->R, tuned ? plan.cps : 0);
+  LaunchGeom g = star_geom(op, tile, nin, op->R, tuned ? plan.cps : 0,
+                           vt<V>::NC == 1 ? real_resident(op, tile) : 0);
   p.nxc = g.nxc;
   p.x_chunk = g.x_chunk;
   if (tile == TILE_SPLIT) {
@@ -769,10 +814,7 @@ inline DirGeom dirs_geom(const gfd_operator* op, int64_t nin) {
   g.ty = (rows + kDirVY - 1) / kDirVY;
   g.gy = (op->n[1] + g.ty * kDirVY - 1) / (g.ty * kDirVY);
   const int64_t tiles = (int64_t)g.gx * g.gy * std::max<int64_t>(nin, 1);
-  const int64_t target = 4LL * num_sms();
-  const int maxc = std::max(1, op->n[0] / std::max(4, 2 * R));
-  const int nxc =
-      (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles));
+  const int nxc = best_chunks(op->n[0], R, tiles, 2LL * num_sms());
   g.x_chunk = (op->n[0] + nxc - 1) / nxc;
   g.nxc = (op->n[0] + g.x_chunk - 1) / g.x_chunk;
   g.bands_per_launch = std::max<int64_t>(1, 65535 / g.nxc);
@@ -930,7 +972,7 @@ inline int64_t partials_count(const gfd_operator* op, int64_t nin) {
   if (op->star) {
     int tile = pick_tile(op);
     TileDims td = tile_dims(tile);
-    LaunchGeom g = star_geom(op, tile, nin, op->R);
+    LaunchGeom g = star_geom(op, tile, nin, op->R, 0, real_resident(op, tile));
     int gx = (op->n[2] + td.BZ - 1) / td.BZ, gy = (op->n[1] + td.BY - 1) / td.BY;
     return (int64_t)gx * gy * g.nxc * nin;
   }

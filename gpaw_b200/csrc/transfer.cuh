@@ -650,6 +650,30 @@ __device__ __forceinline__ V restrict_point_at(const V* __restrict__ base, int X
 #pragma unroll
   for (int j = 0; j < 2 * NN; j++) tz[j] = tr_map(fz - W + 2 * j, p.ni2, p.per2, 1);
   tz[2 * NN] = tr_map(fz, p.ni2, p.per2, 1);
+  if constexpr (NN == 1) {
+    // All 27 loads first (see star_point_at).
+    TrTap tx[3], ty[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      tx[k] = tr_map(fx + k - 1, p.ni0, p.per0, p.ni1 * p.ni2);
+      ty[k] = tr_map(fy + k - 1, p.ni1, p.per1, p.ni2);
+    }
+    V c[3][3][3];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int j = 0; j < 3; j++)
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+          c[i][j][k] = tr_fetch<LD>(base, tx[i], ty[j], tz[k == 1 ? 2 : k >> 1], p);
+    V r = rst_tap<1, V>([&](int ox) {
+      return rst_tap<1, V>([&](int oy) {
+        return rst_tap<1, V>([&](int oz) { return c[ox + 1][oy + 1][oz + 1]; });
+      });
+    });
+    if (p.out_scale != typename vt<V>::S(1)) r = vmul(p.out_scale, r);
+    return r;
+  }
   V v = rst_tap_loop<NN, V>([&](int ox) {
     const TrTap tx = tr_map(fx + ox, p.ni0, p.per0, p.ni1 * p.ni2);
     return rst_tap_loop<NN, V>([&](int oy) {
@@ -663,17 +687,19 @@ __device__ __forceinline__ V restrict_point_at(const V* __restrict__ base, int X
   return v;
 }
 
-// The same at flat index g over all output bands.
-template <class V, int NN, class LD>
-__device__ __forceinline__ V restrict_point(const V* __restrict__ in,
-                                            const TrParams<typename vt<V>::S>& p, long long g) {
-  const long long plane_out = (long long)p.no1 * p.no2;
-  const long long b = g / p.band_out;
-  const long long rem = g - b * p.band_out;
-  const int X = int(rem / plane_out);
-  const int r1 = int(rem - X * plane_out);
-  const int Y = r1 / p.no2, Z = r1 - Y * p.no2;
-  return restrict_point_at<V, NN, LD>(in + b * p.band_in, X, Y, Z, p);
+// Output coordinates of flat index g over all output bands (32-bit arithmetic:
+// fewer than 2^31 points per launch) and its band.
+template <class S>
+__device__ __forceinline__ int tr_split(const TrParams<S>& p, int g, int total, int& X, int& Y,
+                                        int& Z, int& rem) {
+  const int band = int(p.band_out);
+  const int b = total == band ? 0 : g / band;
+  rem = g - b * band;
+  const int row = rem / p.no2;
+  Z = rem - row * p.no2;
+  X = row / p.no1;
+  Y = row - X * p.no1;
+  return b;
 }
 
 // One interpolated point at output coordinates (X, Y, Z), times osc
@@ -704,28 +730,15 @@ __device__ __forceinline__ V interp_point_at(const V* __restrict__ base, const V
   return v;
 }
 
-// The same at flat index g over all output bands.
-template <class V, int NN, bool SUB, class LD>
-__device__ __forceinline__ V interp_point(const V* __restrict__ in, const V* base_out,
-                                          const TrParams<typename vt<V>::S>& p,
-                                          typename vt<V>::S osc, long long g) {
-  const long long plane_out = (long long)p.no1 * p.no2;
-  const long long b = g / p.band_out;
-  const long long rem = g - b * p.band_out;
-  const int X = int(rem / plane_out);
-  const int r1 = int(rem - X * plane_out);
-  const int Y = r1 / p.no2, Z = r1 - Y * p.no2;
-  return interp_point_at<V, NN, SUB, LD>(in + b * p.band_in, SUB ? base_out + g : nullptr, X, Y,
-                                         Z, p, osc);
-}
-
 template <class V, int NN>
 __global__ void __launch_bounds__(256)
 restrict_direct_kernel(const V* __restrict__ in, V* __restrict__ out,
-                       const TrParams<typename vt<V>::S> p, long long total) {
+                       const TrParams<typename vt<V>::S> p, int total) {
   pdl_enter();
-  for (long long g = blockIdx.x * 256LL + threadIdx.x; g < total; g += (long long)gridDim.x * 256) {
-    const V v = restrict_point<V, NN, LoadRO>(in, p, g);
+  for (long long g = blockIdx.x * 256 + threadIdx.x; g < total; g += gridDim.x * 256) {
+    int X, Y, Z, rem;
+    const long long b = tr_split(p, int(g), total, X, Y, Z, rem);
+    const V v = restrict_point_at<V, NN, LoadRO>(in + b * p.band_in, X, Y, Z, p);
     out[g] = v;
     if (p.seed) static_cast<V*>(p.seed)[g] = vmul(p.seed_scale, v);
   }
@@ -734,11 +747,15 @@ restrict_direct_kernel(const V* __restrict__ in, V* __restrict__ out,
 template <class V, int NN, bool SUB>
 __global__ void __launch_bounds__(256)
 interp_direct_kernel(const V* __restrict__ in, V* out, const V* base_out,
-                     const TrParams<typename vt<V>::S> p, long long total) {
+                     const TrParams<typename vt<V>::S> p, int total) {
   pdl_enter();
   const auto osc = out_factor(p);
-  for (long long g = blockIdx.x * 256LL + threadIdx.x; g < total; g += (long long)gridDim.x * 256)
-    out[g] = interp_point<V, NN, SUB, LoadRO>(in, base_out, p, osc, g);
+  for (long long g = blockIdx.x * 256 + threadIdx.x; g < total; g += gridDim.x * 256) {
+    int X, Y, Z, rem;
+    const long long b = tr_split(p, int(g), total, X, Y, Z, rem);
+    out[g] = interp_point_at<V, NN, SUB, LoadRO>(in + b * p.band_in, SUB ? base_out + g : nullptr,
+                                                 X, Y, Z, p, osc);
+  }
 }
 
 }  // namespace gfd

@@ -96,17 +96,26 @@ int restrict1_go(const gfd_transformer* tr, const V* in, V* out, int64_t nin,
 // Outputs (all bands) up to direct_max_points() use the one-thread-per-point
 // forms.
 template <class V, int NN>
-int direct_go(const gfd_transformer* tr, const V* in, V* out, const V* base, int64_t nin,
-                     const TrParams<typename vt<V>::S>& p, cudaStream_t s) {
-  const long long total = p.band_out * nin;
-  long long b = (total + 255) / 256, cap = 8LL * num_sms();
-  const int blocks = int(b < 1 ? 1 : (b > cap ? cap : b));
-  if (!tr->interpolate)
-    launch_k(restrict_direct_kernel<V, NN>, blocks, 256, 0, s, in, out, p, total);
-  else if (base)
-    launch_k(interp_direct_kernel<V, NN, true>, blocks, 256, 0, s, in, out, base, p, total);
-  else
-    launch_k(interp_direct_kernel<V, NN, false>, blocks, 256, 0, s, in, out, nullptr, p, total);
+int transfer_direct_go(const gfd_transformer* tr, const V* in, V* out, const V* base, int64_t nin,
+                       TrParams<typename vt<V>::S> p, cudaStream_t s) {
+  const int64_t most = std::max<int64_t>(1, 2000000000LL / p.band_out);
+  V* seed = static_cast<V*>(p.seed);
+  for (int64_t b0 = 0; b0 < nin; b0 += most) {
+    const int total = int(std::min<int64_t>(most, nin - b0) * p.band_out);
+    const long long b = (total + 255) / 256, cap = 8LL * num_sms();
+    const int blocks = int(b < 1 ? 1 : (b > cap ? cap : b));
+    const V* a = in + b0 * p.band_in;
+    V* o = out + b0 * p.band_out;
+    p.seed = seed ? seed + b0 * p.band_out : nullptr;
+    if (!tr->interpolate)
+      launch_k(restrict_direct_kernel<V, NN>, blocks, 256, 0, s, a, o, p, total);
+    else if (base)
+      launch_k(interp_direct_kernel<V, NN, true>, blocks, 256, 0, s, a, o, base + b0 * p.band_out,
+               p, total);
+    else
+      launch_k(interp_direct_kernel<V, NN, false>, blocks, 256, 0, s, a, o, (const V*)nullptr, p,
+               total);
+  }
   return check_launch("transfer_direct_kernel");
 }
 
@@ -128,12 +137,14 @@ int tr_typed(const gfd_transformer* tr, const void* in, void* out, const void* b
   TunePlan plan;
   const bool tuned = tune_lookup(tr_tune_key(tr, dtype_of<V>(), nin), &plan);
   const int cps = tuned ? plan.cps : 0;
-  if (tuned ? plan.path == PLAN_DIRECT : p.band_out * nin <= direct_max_points()) {
+  // the one-thread-per-point forms index a band with 32 bits
+  const bool small = p.band_in < 2000000000LL && p.band_out < 2000000000LL;
+  if (small && (tuned ? plan.path == PLAN_DIRECT : p.band_out * nin <= direct_max_points())) {
     switch (tr->nn) {
-      case 1: return direct_go<V, 1>(tr, vin, vout, base, nin, p, s);
-      case 2: return direct_go<V, 2>(tr, vin, vout, base, nin, p, s);
-      case 3: return direct_go<V, 3>(tr, vin, vout, base, nin, p, s);
-      case 4: return direct_go<V, 4>(tr, vin, vout, base, nin, p, s);
+      case 1: return transfer_direct_go<V, 1>(tr, vin, vout, base, nin, p, s);
+      case 2: return transfer_direct_go<V, 2>(tr, vin, vout, base, nin, p, s);
+      case 3: return transfer_direct_go<V, 3>(tr, vin, vout, base, nin, p, s);
+      case 4: return transfer_direct_go<V, 4>(tr, vin, vout, base, nin, p, s);
     }
   }
   if (tr->interpolate) {

@@ -9,8 +9,7 @@
 // star_kernel  axis-aligned stencils (Laplace/Gradient on orthorhombic
 //   grids, the reference's cfd case).  A CTA owns a BY x BZ column of
 //   points and marches along axis 0 (the largest stride).  Each thread keeps
-//   a shift register of 2R+1 partial sums for its points; a plane's own
-//   values arrive in registers (prefetched D planes ahead) and contribute to
+//   2R partial sums per point; a plane's own values contribute to
 //   the 2R+1 outputs around it, so x-neighbours are never re-read.  The
 //   in-plane (axis 1 / axis 2) neighbours come from a double-buffered shared
 //   memory tile that the CTA fills with the plane's own values plus a halo

@@ -11,8 +11,9 @@
 //     periodic times the Bloch phase) is staged in shared memory, the axis-2
 //     pass and then the axis-1 pass run there (the reference's pass order,
 //     so the arithmetic matches term by term);
-//   * the axis-0 pass reads a per-thread register queue of the last planes'
-//     2-D results.
+//   * the axis-0 pass works on 2-D results in registers: a queue of the last
+//     planes' (interpolation) or the sums of the coarse planes under way
+//     (restriction).
 // HBM traffic is one read of the input and one write of the output.
 //
 // Weights: Lagrange weights for K = 2*nn taps (c/bmgs/restrict.c:37-57,

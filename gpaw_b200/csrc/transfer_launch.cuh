@@ -13,12 +13,13 @@ namespace gfd {
 template <class V, int NN>
 int restrict_go(const gfd_transformer* tr, const V* in, V* out, int64_t nin,
                        TrParams<typename vt<V>::S>& p, int cps, cudaStream_t s) {
-  // Two coarse rows per thread (16 per CTA) stage fewer halo rows per output
-  // row; complex128 keeps one, so two CTAs still fit on an SM.  Other shapes
-  // measured slower on 256 float64 bands of 112^3 (nn = 3; 2800-2830 GB/s
-  // for this one): 28 columns, which tile 112 exactly, 2580; one coarse row
-  // per thread 2270; 32 rows per CTA 2410; 4 rows per thread 2490 (253
-  // registers); three CTAs per SM (80 registers, spills) 1740.
+  // Two adjacent coarse rows per thread (16 per CTA) stage fewer halo rows per
+  // output row and share axis-1 reads; complex128 keeps one, so two CTAs still
+  // fit on an SM.  256 float64 bands of 224^3 -> 112^3, nn = 3: 3080 GB/s.
+  // Other shapes, measured with the axis-0 queue this kernel had before (2800-2830
+  // for this shape): 28 columns 2580; one coarse row per thread 2270; 32 rows
+  // per CTA 2410; 4 rows per thread 2490 (253 registers); three CTAs per SM (80
+  // registers, spills) 1740.
   constexpr int BZC = 32, TYC = 8, VYC = sizeof(V) >= 16 ? 1 : 2, BYC = TYC * VYC;
   constexpr int W = 2 * NN - 1;
   constexpr int RY = 2 * BYC - 1 + 2 * W, RZ = 2 * BZC - 1 + 2 * W;

@@ -818,7 +818,7 @@ def run_gpu_arm(args):
                          'traffic': traffic, 'algorithmic_bytes_per_launch': nbytes,
                          'kernel': ('star_direct_kernel<cplx<double>,R=3>'
                                     if plan and plan['form'] == 'direct'
-                                    else 'star_kernel<cplx<double>,R=3>')},
+                                    else 'star_pair_kernel (complex128, R=3; 96^3)')},
             'launch_plan': plan,
             'check': check,
             'e2e': e2e,

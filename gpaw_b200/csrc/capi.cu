@@ -244,45 +244,6 @@ extern "C" size_t gfd_last_error(char* buf, size_t len) {
 
 extern "C" const char* gfd_version(void) { return "gpaw-fd-b200 0.1 sm_100a"; }
 
-// Stream-ordered scratch of a few kilobytes for reductions, from a pool of the
-// library's own on each device that keeps up to kScratchKeep bytes across
-// synchronisations.  The default pool gives its memory back whenever the
-// device runs idle, so a call of 40 us paid for mapping it again, about 400 us.
-namespace gfd {
-constexpr uint64_t kScratchKeep = 64ull << 20;
-static int scratch_alloc(double** p, size_t bytes, cudaStream_t s) {
-  static std::mutex mu;
-  static cudaMemPool_t pools[64] = {nullptr};
-  int dev = 0;
-  int st = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
-  if (st) return st;
-  if (dev < 0 || dev >= 64) return set_error(GFD_EUNSUPPORTED, "device index out of range");
-  cudaMemPool_t pool;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (!pools[dev]) {
-      cudaMemPoolProps props = {};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.handleTypes = cudaMemHandleTypeNone;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = dev;
-      cudaMemPool_t np = nullptr;
-      if ((st = check_cuda(cudaMemPoolCreate(&np, &props), "cudaMemPoolCreate(scratch)"))) return st;
-      uint64_t keep = kScratchKeep;
-      if ((st = check_cuda(cudaMemPoolSetAttribute(np, cudaMemPoolAttrReleaseThreshold, &keep),
-                           "cudaMemPoolSetAttribute(scratch)"))) {
-        cudaMemPoolDestroy(np);
-        return st;
-      }
-      pools[dev] = np;
-    }
-    pool = pools[dev];
-  }
-  return check_cuda(cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, pool, s),
-                    "cudaMallocFromPoolAsync(reduction)");
-}
-}  // namespace gfd
-
 extern "C" int gfd_density_interpolate(gfd_transformer* tr, const double* nt_sG, double* nt_sg,
                                        int64_t nspins, double pseudo_charge, double dv_fine,
                                        int renormalize, void* stream) {
@@ -318,7 +279,10 @@ extern "C" int gfd_density_interpolate(gfd_transformer* tr, const double* nt_sG,
   const int64_t n = (int64_t)tr->nin[0] * tr->nin[1] * tr->nin[2] * nspins;
   const int blocks = grid_for(n, kRedThreads, kRedBlocks);
   double* buf = nullptr;
-  if ((st = gfd::scratch_alloc(&buf, sizeof(double) * (kRedBlocks + 1), s))) return st;
+  if ((st = check_cuda(scratch_alloc(reinterpret_cast<void**>(&buf),
+                                     sizeof(double) * (kRedBlocks + 1), s),
+                       "scratch of a reduction")))
+    return st;
   launch_k(interp_sum_kernel, blocks, kRedThreads, 0, s, nt_sG, (long long)n, q, buf);
   st = check_launch("interp_sum_kernel");
   if (!st) st = final_sum_launch(buf, blocks, dv_fine, buf + kRedBlocks, s);
@@ -340,7 +304,9 @@ extern "C" int gfd_grid_sum(const double* a, int64_t n, double scale, double* re
   if (!a) return set_error(GFD_EINVAL, "null array pointer");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   double* buf = nullptr;
-  int st = gfd::scratch_alloc(&buf, sizeof(double) * (kRedBlocks + 1), s);
+  int st = check_cuda(scratch_alloc(reinterpret_cast<void**>(&buf),
+                                    sizeof(double) * (kRedBlocks + 1), s),
+                      "scratch of a reduction");
   if (st) return st;
   st = reduce_launch(GFD_FLOAT64, a, n, false, scale, buf, buf + kRedBlocks, s);
   if (!st)

@@ -28,7 +28,8 @@ struct gfd_operator {
   // component -1, 0 or 1) or their opposites: dirs_kernel's class.
   bool dirs = false;
   // Device scratch of one grid for relaxation (Jacobi ping-pong / frozen
-  // copy for periodic Gauss-Seidel), allocated on first use.
+  // copy for periodic Gauss-Seidel), allocated on first use.  Zero-boundary
+  // Gauss-Seidel does not touch it, so such calls may overlap.
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
   int device = -1;
@@ -141,7 +142,15 @@ int op_launch(const gfd_operator* op, int dtype, int mode, const void* in, void*
 // Number of partial sums op_launch(OP_RESIDUAL) writes for nin bands.
 int64_t op_partials(const gfd_operator* op, int dtype, int mode, int64_t nin);
 
-// Multicolour Gauss-Seidel sweeps (real).  frozen: scratch of one grid.
+// Stream-ordered scratch of one call (scratch.cu), given back with
+// cudaFreeAsync on the same stream; up to kScratchKeep bytes stay mapped.
+constexpr uint64_t kScratchKeep = 64ull << 20;
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+
+// Multicolour Gauss-Seidel sweeps (real).  frozen: scratch of one grid that no
+// other work in flight uses.  A periodic axis needs it (wrapped neighbours are
+// read from a copy of the sweep's start); without one it holds the colour-split
+// copy and may be null (the sweeps then run in phi).
 int op_gs_sweeps(const gfd_operator* op, int dtype, void* phi, const void* rho, int nsweeps,
                  void* frozen, cudaStream_t s);
 int op_gs_colors(const gfd_operator* op);

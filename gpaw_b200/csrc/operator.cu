@@ -96,6 +96,26 @@ static int ensure_scratch(gfd_operator* op, size_t bytes) {
   return GFD_OK;
 }
 
+// Zero-boundary Gauss-Seidel sweeps.  The colour-split copy lives in scratch of
+// this call alone: calls on one operator from different streams or threads may
+// overlap, which they could not in the operator's scratch grid.  No copy while
+// the stream is being captured (the graph would own the allocation), past the
+// bytes that the pool keeps mapped, or when there is no memory for it.
+static int gs_sweeps_own_copy(const gfd_operator* op, int dtype, void* phi, const void* rho,
+                              int nsweeps, size_t bytes, cudaStream_t s) {
+  void* copy = nullptr;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (gs_split_pays(op, op_gs_colors(op)) && bytes <= kScratchKeep &&
+      (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
+       scratch_alloc(&copy, bytes, s) != cudaSuccess)) {
+    cudaGetLastError();
+    copy = nullptr;
+  }
+  const int st = op_gs_sweeps(op, dtype, phi, rho, nsweeps, copy, s);
+  if (copy) cudaFreeAsync(copy, s);
+  return st;
+}
+
 // ---------------------------------------------------------------------------
 // TMA-fed stencil support: the kernel's error flag, the switch, and the
 // tensor maps.
@@ -434,7 +454,10 @@ extern "C" int gfd_operator_relax(gfd_operator* op, int dtype, int relax_method,
   const size_t bytes = (size_t)op->n[0] * op->n[1] * op->n[2] * dtype_size(dtype);
   int st = ensure_scratch(op, bytes);
   if (st) return st;
-  if (relax_method == GFD_RELAX_GS) return op_gs_sweeps(op, dtype, func, source, nrelax, op->scratch, s);
+  if (relax_method == GFD_RELAX_GS)
+    return op->per[0] || op->per[1] || op->per[2]
+               ? op_gs_sweeps(op, dtype, func, source, nrelax, op->scratch, s)
+               : gs_sweeps_own_copy(op, dtype, func, source, nrelax, bytes, s);
   // Weighted Jacobi with w = 0 leaves func unchanged.
   if (w == 0.0) return GFD_OK;
   // Weighted Jacobi: ping-pong between func and the scratch grid.

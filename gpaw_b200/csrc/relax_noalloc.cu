@@ -2,14 +2,15 @@
 // allocate no device memory.
 //
 // gfd_operator_relax needs one grid of device scratch (the second buffer of
-// the Jacobi ping-pong, or the sweep-start copy that periodic Gauss-Seidel
-// reads wrapped neighbours from) and allocates it with cudaMalloc on first
-// use.  Some callers cannot allow that: code running while a CUDA graph is
-// being captured, where an allocation would break or end the capture; hosts
-// that hand the whole device memory to their own pool allocator and forbid
-// other allocations; and real-time loops where an allocation's implicit
-// device synchronisation is not acceptable.  This entry point uses a
-// fixed scratch array compiled into the library instead.
+// the Jacobi ping-pong, the sweep-start copy that periodic Gauss-Seidel
+// reads wrapped neighbours from, or the colour-split copy of large
+// zero-boundary grids) and allocates it.  Some callers cannot allow that:
+// code running while a CUDA graph is being captured, where an allocation
+// would break or end the capture; hosts that hand the whole device memory to
+// their own pool allocator and forbid other allocations; and real-time loops
+// where an allocation's implicit device synchronisation is not acceptable.
+// This entry point uses a fixed scratch array compiled into the library
+// instead.
 //
 // The scratch is a file-scope __device__ array of kNoAllocScratchBytes
 // (16 MiB: up to 2,097,152 float64 points, a 128^3 grid, or 4,194,304

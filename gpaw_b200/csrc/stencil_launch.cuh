@@ -1034,6 +1034,11 @@ int gs_sweeps(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* froz
 // The same on a colour-split copy in the scratch grid, from kGsSplitPoints
 // points of a zero-boundary grid up.
 constexpr long long kGsSplitPoints = 40000;
+inline bool gs_split_pays(const gfd_operator* op, int ncolor) {
+  return op->star && !op->per[0] && !op->per[1] && !op->per[2] && (op->R == 2 || op->R == 3) &&
+         ncolor == op->R + 1 &&
+         (long long)op->n[0] * op->n[1] * op->n[2] >= kGsSplitPoints;
+}
 template <class V, int R>
 int gs_split_sweeps(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* copy,
                     const StarParams<typename vt<V>::S>& p, cudaStream_t s) {
@@ -1056,11 +1061,9 @@ int gs_typed(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* froze
   if (op->star) {
     StarParams<S> p;
     gs_star_params(op, p);
-    if (!op->per[0] && !op->per[1] && !op->per[2] && p.band >= kGsSplitPoints && nsweeps > 0 &&
-        ncolor == op->R + 1) {
-      if (op->R == 2) return gs_split_sweeps<V, 2>(op, phi, rho, nsweeps, frozen, p, s);
-      if (op->R == 3) return gs_split_sweeps<V, 3>(op, phi, rho, nsweeps, frozen, p, s);
-    }
+    if (frozen && nsweeps > 0 && gs_split_pays(op, ncolor))
+      return op->R == 2 ? gs_split_sweeps<V, 2>(op, phi, rho, nsweeps, frozen, p, s)
+                        : gs_split_sweeps<V, 3>(op, phi, rho, nsweeps, frozen, p, s);
     switch (op->R) {
       case 1: return gs_sweeps<V, 1>(op, phi, rho, nsweeps, frozen, ncolor, p, s);
       case 2: return gs_sweeps<V, 2>(op, phi, rho, nsweeps, frozen, ncolor, p, s);

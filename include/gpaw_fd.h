@@ -109,7 +109,9 @@ GFD_API int gfd_operator_apply(gfd_operator* op, int dtype, const void* in, void
  * is a sequential sweep; it is replaced by multicolour Gauss-Seidel
  * ((i0+i1+i2) mod (range+1) colours, a valid colouring for axis-aligned
  * stencils), compared by the converged result, not by iterates.
- * Uses a device scratch array of one grid owned by the operator. */
+ * Jacobi sweeps and Gauss-Seidel sweeps with a periodic axis use a device
+ * scratch array of one grid owned by the operator: such calls on one operator
+ * must not overlap on the GPU.  Zero-boundary Gauss-Seidel calls may. */
 GFD_API int gfd_operator_relax(gfd_operator* op, int dtype, int relax_method, void* func,
                        const void* source, int nrelax, double w, void* stream);
 

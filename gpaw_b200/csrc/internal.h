@@ -146,6 +146,9 @@ int64_t op_partials(const gfd_operator* op, int dtype, int mode, int64_t nin);
 // cudaFreeAsync on the same stream; up to kScratchKeep bytes stay mapped.
 constexpr uint64_t kScratchKeep = 64ull << 20;
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+// Id of the context that this thread's CUDA calls work in, unique in the life
+// of the process (scratch.cu); 0 if there is none.
+unsigned long long context_id();
 
 // Multicolour Gauss-Seidel sweeps (real).  frozen: scratch of one grid that no
 // other work in flight uses.  A periodic axis needs it (wrapped neighbours are

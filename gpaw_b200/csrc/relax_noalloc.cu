@@ -33,50 +33,28 @@ constexpr size_t kNoAllocScratchBytes = size_t(16) << 20;
 
 static __device__ __align__(256) unsigned char g_relax_scratch[kNoAllocScratchBytes];
 
-// Per device: the context the address was looked up in and the address.
+// Per device: the context (its id) the address was looked up in and the address.
 struct ScratchAddr {
-  void* ctx = nullptr;
+  unsigned long long ctx = 0;
   void* addr = nullptr;
 };
 static ScratchAddr g_scratch_addr[64];
 static std::mutex g_scratch_mutex;
-
-// The current context (CUcontext, as void*) through the driver entry point,
-// so the library needs no link-time dependency on libcuda.
-typedef int (*CtxGetCurrentFn)(void**);
-static int current_context(void** ctx) {
-  static CtxGetCurrentFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<CtxGetCurrentFn>(f);
-  }();
-  if (!fn) return set_error(GFD_ECUDA, "cuCtxGetCurrent is not available");
-  *ctx = nullptr;
-  if (fn(ctx) != 0 || !*ctx) return set_error(GFD_ECUDA, "no current CUDA context");
-  return GFD_OK;
-}
 
 static int scratch_for_current_device(void** out) {
   int dev = 0;
   int st = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
   if (st) return st;
   if (dev < 0 || dev >= 64) return set_error(GFD_EUNSUPPORTED, "device index out of range");
+  const unsigned long long ctx = context_id();
+  if (ctx == 0) return set_error(GFD_ECUDA, "no current CUDA context");
   std::lock_guard<std::mutex> lock(g_scratch_mutex);
   ScratchAddr& e = g_scratch_addr[dev];
-  void* ctx = nullptr;
-  // No current context yet (a first call before any other CUDA work on this
-  // thread) reads as "not cached": the lookup below makes the runtime bind
-  // the device's primary context, which is then recorded.
-  if (current_context(&ctx) != GFD_OK) ctx = nullptr;
-  if (!e.addr || !ctx || e.ctx != ctx) {
+  if (!e.addr || e.ctx != ctx) {
     void* p = nullptr;
     st = check_cuda(cudaGetSymbolAddress(&p, g_relax_scratch),
                     "cudaGetSymbolAddress(relaxation scratch)");
     if (st) return st;
-    if ((st = current_context(&ctx))) return st;
     e.ctx = ctx;
     e.addr = p;
   }

@@ -144,3 +144,36 @@ def test_noalloc_relax_size_limit(cuda):
     phi64 = torch.zeros((150,) * 3, dtype=torch.float64, device=cuda)
     assert _call(_lib.lib.gfd_operator_relax_noalloc, op, _lib.GFD_FLOAT64, phi64, phi64,
                  _lib.GFD_RELAX_JACOBI, 1, 1.0, null) == _lib.GFD_EINVAL
+
+
+def test_reductions_after_a_device_reset(cuda):
+    """gfd_grid_sum keeps its scratch in a pool of its own; after
+    cudaDeviceReset (in a process of its own) the next call makes a new one."""
+    import subprocess
+    import sys
+    import textwrap
+    pytest.importorskip('cuda.bindings.runtime')
+    from gpaw_b200 import _lib
+    child = textwrap.dedent("""
+        import ctypes
+        import numpy as np
+        from cuda.bindings import runtime as rt
+        lib = ctypes.CDLL(%r)
+        a = np.arange(1000.0)
+        for turn in range(3):
+            err, p = rt.cudaMalloc(a.nbytes)
+            assert err == rt.cudaError_t.cudaSuccess, err
+            err, = rt.cudaMemcpy(p, a.ctypes.data, a.nbytes,
+                                 rt.cudaMemcpyKind.cudaMemcpyHostToDevice)
+            assert err == rt.cudaError_t.cudaSuccess, err
+            for call in range(2):
+                r = ctypes.c_double()
+                status = lib.gfd_grid_sum(ctypes.c_void_p(p), ctypes.c_int64(1000),
+                                          ctypes.c_double(2.0), ctypes.byref(r), None)
+                assert status == 0 and r.value == 999000.0, (turn, call, status, r.value)
+            err, = rt.cudaDeviceReset()
+            assert err == rt.cudaError_t.cudaSuccess, err
+    """) % _lib.LIB_PATH
+    got = subprocess.run([sys.executable, '-c', child], capture_output=True, text=True,
+                         timeout=300)
+    assert got.returncode == 0, got.stdout + got.stderr

@@ -931,6 +931,7 @@ int launch_general_typed(const gfd_operator* op, int mode, const void* in, void*
                          const void* rho, int64_t nin, const double* phase_cd, double w,
                          double* partials, cudaStream_t s) {
   using S = typename vt<V>::S;
+  if (op->ncoefs > kMaxCoefs) return set_error(GFD_EUNSUPPORTED, "too many stencil coefficients");
   if (dirs_eligible(op, mode)) {
     const V* a = static_cast<const V*>(in);
     V* b = static_cast<V*>(out);
@@ -942,7 +943,6 @@ int launch_general_typed(const gfd_operator* op, int mode, const void* in, void*
     if (mode == OP_RESIDUAL)
       return dirs_dispatch<V, MODE_RESIDUAL>(op, mode, a, b, r, nin, phase_cd, w, partials, s);
   }
-  if (op->ncoefs > kMaxCoefs) return set_error(GFD_EUNSUPPORTED, "too many stencil coefficients");
   GenParams<S> p{};
   p.n0 = op->n[0]; p.n1 = op->n[1]; p.n2 = op->n[2];
   p.per0 = op->per[0]; p.per1 = op->per[1]; p.per2 = op->per[2];

@@ -259,3 +259,17 @@ def test_timer_nesting_and_metrics_log(tmp_path):
     recs = [json.loads(line) for line in open(path)]
     assert recs[0]['kind'] == 'request' and recs[0]['N'] == 32 and recs[0]['residual'] == 1e-11
     assert [r['region'] for r in recs[1:]] == ['SCF', 'SCF.Poisson', 'Other', 'Total']
+
+
+def test_coefficient_limit_holds_for_every_stencil_class():
+    """128 coefficients at most with cross terms, also where the offsets are
+    multiples of lattice directions; refused before anything is launched."""
+    from gpaw_b200 import _lib
+    offs = [(0, 0, 0)] + [(1, 1, 0), (-1, -1, 0)] * 64
+    st, h = _create_op(np.ones(len(offs)), offs, (8, 8, 8))
+    assert st == _lib.GFD_OK
+    buf = (ctypes.c_double * 1024)()
+    st = _lib.lib.gfd_operator_apply(h, _lib.GFD_FLOAT64, ctypes.addressof(buf),
+                                     ctypes.addressof(buf) + 4096, 1, None, None)
+    assert st == _lib.GFD_EUNSUPPORTED and 'coefficients' in _lib.last_error()
+    assert _lib.lib.gfd_operator_destroy(h) == 0

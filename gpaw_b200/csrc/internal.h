@@ -20,12 +20,14 @@ struct gfd_operator {
   int cfd = 1;
   // Axis-aligned decomposition (star stencils).
   bool star = false;
+  bool full_star = false;  // with all 6 R neighbours
   int R = 0;
   double c0 = 0.0;
   double cx[13] = {0}, cy[13] = {0}, cz[13] = {0};  // index 6 + k
   double diag = 0.0;     // weight of the zero offset
   // Every offset is k d with d one of the 13 lattice directions (every
-  // component -1, 0 or 1) or their opposites: dirs_kernel's class.
+  // component -1, 0 or 1) or their opposites, and each d that occurs has all
+  // k = 1 .. mp: dirs_kernel's class.
   bool dirs = false;
   // Device scratch of one grid for relaxation (Jacobi ping-pong / frozen
   // copy for periodic Gauss-Seidel), allocated on first use.  Zero-boundary

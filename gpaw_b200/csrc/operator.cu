@@ -369,15 +369,21 @@ extern "C" int gfd_operator_create(int ncoefs, const double* coefs, const int64_
   for (int c = 0; c < ncoefs; c++)
     if (op->off[3 * c] == 0 && op->off[3 * c + 1] == 0 && op->off[3 * c + 2] == 0)
       op->diag = coefs[c];
-  op->dirs = mp >= 1;
-  for (int c = 0; c < ncoefs; c++) {
-    int m = 0;
-    for (int a = 0; a < 3; a++) m = std::max(m, std::abs(op->off[3 * c + a]));
-    for (int a = 0; a < 3; a++) {
-      const int o = std::abs(op->off[3 * c + a]);
-      if (o != 0 && o != m) op->dirs = false;
-    }
+  // Which multiples of each signed lattice direction occur.  dirs_kernel takes a
+  // direction whole, so one with a gap stays with general_kernel: its missing
+  // weights would turn an infinity that the stencil does not reach into a NaN.
+  op->dirs = mp >= 1 && mp < 16;
+  unsigned seen[27] = {0};
+  for (int c = 0; c < ncoefs && op->dirs; c++) {
+    const int* o = &op->off[3 * c];
+    const int m = std::max(std::abs(o[0]), std::max(std::abs(o[1]), std::abs(o[2])));
+    if (m == 0) continue;
+    for (int a = 0; a < 3; a++)
+      if (o[a] != 0 && std::abs(o[a]) != m) op->dirs = false;
+    if (op->dirs) seen[9 * (o[0] / m) + 3 * (o[1] / m) + o[2] / m + 13] |= 1u << m;
   }
+  for (unsigned d : seen)
+    if (d != 0 && d != (2u << mp) - 2u) op->dirs = false;
   // Axis-aligned decomposition.
   bool star = mp <= kMaxR;
   for (int c = 0; c < ncoefs && star; c++) {
@@ -396,6 +402,15 @@ extern "C" int gfd_operator_create(int ncoefs, const double* coefs, const int64_
     op->R = std::max(mp, 1);
   }
   op->star = star;
+  op->full_star = star && mp >= 1;
+  for (int k = 1; k <= mp && op->full_star; k++)
+    for (int a = 0; a < 3; a++)
+      for (int sgn = -1; sgn <= 1; sgn += 2) {
+        bool have = false;
+        for (int c = 0; c < ncoefs; c++)
+          have = have || (op->off[3 * c + a] == sgn * k);
+        if (!have) op->full_star = false;
+      }
   *out = op;
   return GFD_OK;
 }

@@ -1,6 +1,7 @@
-// stencil_dirs.cuh -- stencils whose offsets are multiples k d, k = 1 .. R, of
-// the 13 lattice directions d (every component -1, 0 or 1): the Laplacians of
-// non-orthogonal cells (gpaw/fd_operators.py:231-282) and the Mehrstellen pair.
+// stencil_dirs.cuh -- stencils whose offsets are the multiples k d, all of
+// k = 1 .. R, of lattice directions d (every component -1, 0 or 1; 13 and their
+// opposites): the Laplacians of non-orthogonal cells
+// (gpaw/fd_operators.py:231-282) and the Mehrstellen pair.
 //
 // A CTA marches a tile along axis 0 as star_kernel does; planes arrive with
 // their full halo (corners included) in a cp.async ring.  On an incoming plane
@@ -44,7 +45,8 @@ struct DirParams {
   S wx[2 * kDirMaxR + 1];
   S w[8][kDirMaxR][3];
   unsigned mask;       // bit 3 h + i: weights w[h][.][i] exist
-  S c0;                // MODE_JACOBI: the folded centre weight is in wx
+  unsigned xmask;      // bit 0: the centre's weight exists, 1: those of
+                       // +1 .. +R planes, 2: of -1 .. -R planes
   S wc;                // MODE_JACOBI: +-w / diagonal
   int fix_yz;
   Phases<S> P;
@@ -185,8 +187,16 @@ dirs_kernel(const V* __restrict__ in, V* __restrict__ out, const V* __restrict__
 #pragma unroll
       for (int j = 0; j < VY; j++) {
         const V v = at(j, 0, 0);
+        // no weight, no product: zero times an infinity is not zero
+        if (p.xmask & 1u) madd(acc[j][R], p.wx[kDirMaxR], v);
+        if (p.xmask & 2u) {
 #pragma unroll
-        for (int dx = -R; dx <= R; dx++) madd(acc[j][R - dx], p.wx[kDirMaxR + dx], v);
+          for (int dx = 1; dx <= R; dx++) madd(acc[j][R - dx], p.wx[kDirMaxR + dx], v);
+        }
+        if (p.xmask & 4u) {
+#pragma unroll
+          for (int dx = 1; dx <= R; dx++) madd(acc[j][R + dx], p.wx[kDirMaxR - dx], v);
+        }
       }
 #pragma unroll
       for (int h = 0; h < 8; h++) {

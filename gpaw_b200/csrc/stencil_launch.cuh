@@ -838,6 +838,7 @@ void dirs_params(const gfd_operator* op, int mode, double w, const double* phase
     if (jacobi && c == 0) x = -(1.0 - w) * x / w;
     if (dy == 0 && dz == 0) {
       wx[kDirMaxR + dx] += x;
+      p.xmask |= dx == 0 ? 1u : dx > 0 ? 2u : 4u;
       continue;
     }
     const int k = std::max(std::abs(dy), std::abs(dz));
@@ -1035,7 +1036,7 @@ int gs_sweeps(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* froz
 // points of a zero-boundary grid up.
 constexpr long long kGsSplitPoints = 40000;
 inline bool gs_split_pays(const gfd_operator* op, int ncolor) {
-  return op->star && !op->per[0] && !op->per[1] && !op->per[2] && (op->R == 2 || op->R == 3) &&
+  return op->full_star && !op->per[0] && !op->per[1] && !op->per[2] && (op->R == 2 || op->R == 3) &&
          ncolor == op->R + 1 &&
          (long long)op->n[0] * op->n[1] * op->n[2] >= kGsSplitPoints;
 }
@@ -1058,7 +1059,9 @@ template <class V>
 int gs_typed(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V* frozen, int ncolor,
              cudaStream_t s) {
   using S = typename vt<V>::S;
-  if (op->star) {
+  // The star form multiplies all 6 R weights; an operator that lacks some keeps
+  // the offset table, which touches only the neighbours that there are.
+  if (op->full_star) {
     StarParams<S> p;
     gs_star_params(op, p);
     if (frozen && nsweeps > 0 && gs_split_pays(op, ncolor))

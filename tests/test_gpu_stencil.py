@@ -317,6 +317,73 @@ def test_non_finite_values_stay_within_reach(cuda, where, value):
             assert torch.equal(bad, want)
 
 
+def reach(gd, offsets, where):
+    """The points whose stencil holds grid point `where`."""
+    want = np.zeros(tuple(gd.n_c), bool)
+    for off in offsets:
+        p = [w - int(d) for w, d in zip(where, off)]
+        if all(per or 0 <= x < m for x, m, per in zip(p, want.shape, gd.pbc_c)):
+            want[tuple(x % m for x, m in zip(p, want.shape))] = True
+    return want
+
+
+# Offset sets with and without a centre, an axis-0 column, opposites, and
+# distances short of the range.
+GAPPED = [[(0, 0, 0), (3, 3, 0), (-3, -3, 0), (0, 1, 1)],
+          [(0, 1, -1), (0, 2, -2), (0, 3, -3)],
+          [(0, 0, 0), (1, 1, 1), (2, 2, 2), (3, 3, 3), (1, 0, 0), (2, 0, 0), (3, 0, 0)],
+          [(0, 0, 0), (0, 1, 1), (0, -1, -1), (-2, 0, 2), (2, 0, -2)]]
+
+
+@pytest.mark.parametrize('offs', GAPPED)
+@pytest.mark.parametrize('where', [(5, 6, 7), (0, 0, 0), (19, 11, 25)])
+def test_non_finite_values_and_lattice_directions(cuda, offs, where):
+    """Offsets with cross terms: an infinity reaches the outputs whose stencil
+    holds it and no others; finite inputs match the oracle."""
+    import torch
+    from gpaw_b200.fd_operators import FDOperator
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    args = ((20, 12, 26), np.array((20, 12, 26)) * 0.25, (1, 0, 1))
+    gd = GridDescriptor(*args)
+    where = tuple(min(w, int(n) - 1) for w, n in zip(where, gd.n_c))
+    coefs = np.linspace(0.5, 1.5, len(offs))
+    rng = np.random.default_rng(3)
+    a = rng.standard_normal((2,) + tuple(gd.n_c))
+    assert rel_err(gpu_apply(cuda, args, coefs, offs, a), K.fd_apply(coefs, offs, gd.pbc_c, a)) < TOL
+    for dtype in (float, complex):
+        x = np.zeros((2,) + tuple(gd.n_c), dtype)
+        x[(1,) + where] = np.inf
+        got = gpu_apply(cuda, args, coefs, offs, x)
+        assert np.isfinite(got[0]).all()
+        assert np.array_equal(~np.isfinite(got[1]), reach(gd, offs, where))
+
+
+def test_gauss_seidel_without_some_neighbours(cuda):
+    """A stencil along two axes: an infinity on another row stays there, and
+    finite sweeps match the colour-by-colour reference."""
+    import torch
+    from gpaw_b200.fd_operators import FDOperator
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    N = (36, 35, 37)
+    gd = GridDescriptor(N, tuple(0.3 * x for x in N), False)
+    offs = [(0, 0, 0)] + [tuple(s * k * np.eye(3, dtype=int)[a]) for a in (0, 2) for k in (1, 2)
+                          for s in (1, -1)]
+    coefs = np.array([-8.0] + [1.2, 1.2, -0.1, -0.1] * 2)
+    op = FDOperator(coefs, offs, gd, float)
+    rng = np.random.default_rng(5)
+    phi, rho = (rng.standard_normal(tuple(gd.n_c)) for _ in range(2))
+    t = dev(phi, cuda)
+    op.relax(1, t, dev(rho, cuda), 2)
+    ref = multicolour_gs_reference(np.array(coefs), np.array(offs), gd.pbc_c, phi, rho, 2)
+    assert rel_err(host(t), ref) < TOL
+    phi[:, 20, :] = np.inf
+    t = dev(phi, cuda)
+    op.relax(1, t, dev(rho, cuda), 1)
+    got = host(t)
+    rest = [y for y in range(got.shape[1]) if y != 20]
+    assert np.isfinite(got[:, rest]).all()
+
+
 DIRECTION_GRIDS = [((4, 4, 4), 1), ((6, 11, 49), (1, 0, 1)), ((9, 50, 48), 1), ((17, 7, 97), 0),
                    ((8, 130, 5), (0, 1, 1))]
 

@@ -262,13 +262,9 @@ extern "C" int gfd_density_interpolate(gfd_transformer* tr, const double* nt_sG,
   // The integral of the result comes from the coarse values (interp_sum_kernel),
   // so the interpolation writes the renormalised density at once: 2 spins of
   // 64 x 64 x 72, nn = 3, 57 us when the result was summed and scaled.
-  static const double kLag[4][4] = {{0.5},
-                                    {0.5625, -0.0625},
-                                    {0.5859375, -0.09765625, 0.01171875},
-                                    {0.59814453125, -0.11962890625, 0.02392578125, -0.00244140625}};
   InterpSum q{};
   q.nn = tr->nn;
-  for (int k = 0; k < tr->nn; k++) q.w[k] = kLag[tr->nn - 1][k];
+  lagrange_weights(tr->nn, q.w);
   for (int c = 0; c < 3; c++) {
     q.n[c] = tr->nin[c];
     q.nf[c] = tr->nout[c];
@@ -283,7 +279,10 @@ extern "C" int gfd_density_interpolate(gfd_transformer* tr, const double* nt_sG,
                                      sizeof(double) * (kRedBlocks + 1), s),
                        "scratch of a reduction")))
     return st;
-  launch_k(interp_sum_kernel, blocks, kRedThreads, 0, s, nt_sG, (long long)n, q, buf);
+  if (n < 2000000000)  // the last step of the loop stays below 2^31
+    launch_k(interp_sum_kernel<int>, blocks, kRedThreads, 0, s, nt_sG, (int)n, q, buf);
+  else
+    launch_k(interp_sum_kernel<long long>, blocks, kRedThreads, 0, s, nt_sG, (long long)n, q, buf);
   st = check_launch("interp_sum_kernel");
   if (!st) st = final_sum_launch(buf, blocks, dv_fine, buf + kRedBlocks, s);
   if (!st)

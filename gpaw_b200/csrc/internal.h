@@ -174,6 +174,8 @@ int tr_launch_ex(const gfd_transformer* tr, int dtype, const void* in, void* out
                  const void* base, int64_t nin, const double* phases, double out_scale,
                  void* seed, double seed_scale, cudaStream_t s, const double* total = nullptr,
                  double target = 0.0);
+// Weights of the 2 nn-point interpolation by distance, nearest first.
+void lagrange_weights(int nn, double w[4]);
 // Interpolation with the correction fused: out = base - interpolate(in)
 // (in place when base == out).
 int tr_launch_sub(const gfd_transformer* tr, int dtype, const void* in, void* out,

@@ -25,9 +25,8 @@
 
 namespace gfd {
 
-template <int NN, class S> __device__ __forceinline__ S lagw(int m);
 template <int NN, class S>
-__device__ __forceinline__ S lagw(int m) {
+__host__ __device__ __forceinline__ S lagw(int m) {
   if (NN == 1) return S(0.5);
   if (NN == 2) return m == 0 ? S(0.5625) : S(-0.0625);
   if (NN == 3) return m == 0 ? S(0.58593750) : (m == 1 ? S(-0.09765625) : S(0.01171875));

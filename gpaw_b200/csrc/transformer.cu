@@ -36,6 +36,14 @@ int tr_launch_ex(const gfd_transformer* tr, int dtype, const void* in, void* out
   return set_error(GFD_EINVAL, "unknown dtype");
 }
 
+void lagrange_weights(int nn, double w[4]) {
+  for (int k = 0; k < nn; k++)
+    w[k] = nn == 1   ? lagw<1, double>(k)
+           : nn == 2 ? lagw<2, double>(k)
+           : nn == 3 ? lagw<3, double>(k)
+                     : lagw<4, double>(k);
+}
+
 int tr_launch_sub(const gfd_transformer* tr, int dtype, const void* in, void* out,
                   const void* base, int64_t nin, const double* phases, cudaStream_t s) {
   return tr_launch_ex(tr, dtype, in, out, base, nin, phases, 1.0, nullptr, 0.0, s);

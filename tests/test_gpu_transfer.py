@@ -157,6 +157,60 @@ def test_pseudo_density_interpolation(cuda, pbc):
         assert abs(of.integrate(host(out)).sum() - pseudo_charge) < 1e-12
 
 
+# Both forms of the interpolation (a point per thread up to 300000 fine points),
+# every order, and axes so short that both edges cut one point's weights.
+DENSITY_GRIDS = [((12, 10, 14), 0, 1), ((40, 36, 44), (0, 1, 0), 1), ((12, 10, 14), (1, 0, 1), 2),
+                 ((40, 36, 44), 0, 2), ((44, 36, 40), (0, 0, 1), 3), ((64, 64, 72), 0, 3),
+                 ((12, 12, 14), 0, 4), ((40, 36, 44), (1, 1, 0), 4), ((64, 48, 4), 0, 1),
+                 ((64, 48, 4), 0, 3), ((64, 48, 5), (1, 0, 0), 4)]
+
+
+@pytest.mark.parametrize('N,pbc,nn', DENSITY_GRIDS)
+def test_renormalised_density_forms(cuda, N, pbc, nn):
+    """The factor that the interpolation applies, from the coarse values, is the
+    pseudo charge over the integral of the oracle's interpolation."""
+    import torch
+    from gpaw_b200.density import interpolate_pseudo_density
+    from gpaw_b200.transformers import Transformer
+    og = G.Grid(N, tuple(0.35 * n for n in N), pbc)
+    of = og.refine()
+    gd = product_grid(og)
+    fine = gd.refine()
+    nt = np.random.default_rng(nn).uniform(0, 1, (2,) + tuple(og.n_c))
+    ref = K.transform(og, of, nn, nt, nthreads=8)
+    ref = ref * (2.5 / of.integrate(ref).sum())
+    out = torch.empty((2,) + tuple(int(x) for x in fine.n_c), dtype=torch.float64, device=cuda)
+    interpolate_pseudo_density(Transformer(gd, fine, nn), dev(nt, cuda), out, fine, 2.5)
+    assert rel_err(host(out), ref) < TOL
+
+
+@pytest.mark.parametrize('k,pad,skip,size', [(2, (2, 3), (0, 0), 8), (6, (2, 3), (1, 0), 9),
+                                             (6, (5, 4), (0, 1), 12), (4, (0, 3), (1, 1), 10)])
+def test_renormalised_density_of_other_layouts(cuda, k, pad, skip, size):
+    """Interpolations of more or less than one period, through the C interface:
+    the result is the plain interpolation times charge / (dv sum)."""
+    import ctypes
+    import torch
+    from gpaw_b200 import _lib
+    fine = 2 * (size + sum(pad) - (k - 1) + skip[1]) - sum(skip)
+    h = _lib._vp()
+    arg = [_lib.i64(x) for x in ([size] * 3, [fine] * 3, list(pad) * 3, [0] * 6, list(skip) * 3,
+                                 [0] * 6)]
+    _lib.check(_lib.lib.gfd_transformer_create(arg[0][1], arg[1][1], k, arg[2][1], arg[3][1],
+                                               arg[4][1], arg[5][1], 1, 1, ctypes.byref(h)))
+    a = torch.rand((2,) + (size,) * 3, dtype=torch.float64, device=cuda)
+    plain = torch.empty((2,) + (fine,) * 3, dtype=torch.float64, device=cuda)
+    out = torch.empty_like(plain)
+    stream = torch.cuda.current_stream().cuda_stream
+    _lib.check(_lib.lib.gfd_transformer_apply(h, _lib.GFD_FLOAT64, a.data_ptr(), plain.data_ptr(),
+                                              2, None, stream))
+    _lib.check(_lib.lib.gfd_density_interpolate(h, a.data_ptr(), out.data_ptr(), 2, 4.0, 0.01, 1,
+                                                stream))
+    ref = host(plain)
+    assert rel_err(host(out), ref * (4.0 / (0.01 * ref.sum()))) < TOL
+    _lib.check(_lib.lib.gfd_transformer_destroy(h))
+
+
 _RESTRICT_SCRIPT = r'''
 import json, sys
 import numpy as np

@@ -148,10 +148,11 @@ constexpr size_t star_smem_bytes() {
 //    outside this CTA's axis-0 chunk are copied without their halo.
 //  * Axis-1 neighbours and the own values come from one column read of
 //    VY+2R cells; axis-2 neighbours from 2R reads per point.
-//  * Axis 0: each point keeps 2R partial sums in registers; plane p adds its
-//    own value into the sums of outputs p-R..p+R (output p-R is stored before
-//    its slot starts output p+R).  The plane loop is unrolled by 2R so the ring
-//    index of every sum is a compile-time constant.
+//  * Axis 0: each point keeps 2R + 1 partial sums in registers; plane p adds
+//    its own value into the sums of outputs p-R..p+R.  The plane loop is
+//    unrolled by the number of sums, so the ring index of every sum is a
+//    compile-time constant.  LOW: 2R sums (output p-R is stored before its slot
+//    starts output p+R), fewer registers and a longer chain per plane.
 //  * MODE_JACOBI folds the (1-w) phi term into the centre weight:
 //    phi_new = (w/c0) (rho - sum_{p>=1} c_p phi_p - c0' phi) with
 //    c0' = -(1-w) c0 / w, which equals (1-w) phi + w (rho - sum) / c0.
@@ -165,19 +166,16 @@ constexpr size_t star_smem_bytes() {
 // there) and 3232 at 2; the 48-column tile at 2 per SM 4010-4099, at 3
 // (spilling) 2770.
 constexpr int kShortTileZ = 32, kTile48Z = 48;
-// The 32 x 4-thread tile with 4 rows each (8-byte and smaller values) runs four
-// CTAs per SM up to radius 3 (128 registers): a 127^3 float64 Jacobi sweep, whose
-// 608 CTAs are then resident at once, took 18.8 us against 23.5 us with three; 128 bands of 96^3 the same 4120 GB/s
-// either way.
-template <int BZ, int TY, int VY, int R, int BYTES, int MODE>
+// LOW forms: four CTAs per SM of the 32 x 4-thread tile with 4 rows each (128
+// registers), three of the 48 x 4-thread one.
+template <int BZ, int TY, int VY, bool LOW>
 constexpr int star_min_ctas() {
-  if (TY == 4 && VY == 2) return BZ == kShortTileZ ? 3 : (BZ == kTile48Z ? 2 : 1);
-  if (TY == 4 && VY == 4 && R <= 3 && BYTES <= 8) return BZ == 32 ? 4 : (BZ == kTile48Z ? 3 : 1);
-  return 1;
+  if (LOW) return BZ == kTile48Z ? 3 : 4;
+  return TY == 4 && VY == 2 ? (BZ == kShortTileZ ? 3 : (BZ == kTile48Z ? 2 : 1)) : 1;
 }
 
-template <class V, int R, int BZ, int TY, int VY, int S, int MODE>
-__global__ void __launch_bounds__(BZ * TY, star_min_ctas<BZ, TY, VY, R, sizeof(V), MODE>())
+template <class V, int R, int BZ, int TY, int VY, int S, int MODE, bool LOW>
+__global__ void __launch_bounds__(BZ * TY, star_min_ctas<BZ, TY, VY, LOW>())
 star_kernel(const V* __restrict__ in, V* __restrict__ out, const V* __restrict__ rho,
             const StarParams<typename vt<V>::S> p) {
   pdl_enter();
@@ -185,7 +183,7 @@ star_kernel(const V* __restrict__ in, V* __restrict__ out, const V* __restrict__
   constexpr int NT = BZ * TY, BY = TY * VY;
   constexpr int SY = BY + 2 * R, SZ = BZ + 2 * R, CELLS = SY * SZ;
   constexpr int CPT = (CELLS + NT - 1) / NT;
-  constexpr int Q = 2 * R;
+  constexpr int Q = LOW ? 2 * R : 2 * R + 1;
   constexpr bool RHO = MODE == MODE_JACOBI || MODE == MODE_RESIDUAL;
   constexpr bool POT = MODE == MODE_POTENTIAL;
   constexpr int RCELLS = RHO ? BY * BZ : 0;
@@ -398,13 +396,14 @@ star_kernel(const V* __restrict__ in, V* __restrict__ out, const V* __restrict__
             for (int k = 1; k <= R; k++)
               madd(acc[j][(u - k + 2 * Q) % Q], p.cx[kMaxR + k], own[j]);  // output pl-k: offset +k
 #pragma unroll
-            for (int k = 1; k < R; k++)
+            for (int k = 1; k <= (LOW ? R - 1 : R); k++)
               madd(acc[j][(u + k) % Q], p.cx[kMaxR - k], own[j]);  // output pl+k: offset -k
           }
         }
 
         const int q = pl - R;
-        const int qs = (u + R) % Q;  // slot of output pl - R, then of output pl + R
+        // slot of output pl - R, then of output pl + R (LOW) or pl + R + 1
+        const int qs = (u - R + 2 * Q) % Q;
         if (q >= x0 && q < x1) {
           const V* rt = rtiles + st * RCELLS + ty * VY * BZ + tz;
           char* dstp = out_c + size_t(q) * plane_b;
@@ -426,7 +425,7 @@ star_kernel(const V* __restrict__ in, V* __restrict__ out, const V* __restrict__
         }
 #pragma unroll
         for (int j = 0; j < VY; j++)
-          acc[j][qs] = xs >= 0 ? vmul(p.cx[kMaxR - R], own[j]) : vzero<V>();
+          acc[j][qs] = LOW && xs >= 0 ? vmul(p.cx[kMaxR - R], own[j]) : vzero<V>();
       }
     }
   }

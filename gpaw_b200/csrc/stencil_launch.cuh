@@ -116,11 +116,17 @@ inline LaunchGeom star_geom(const gfd_operator* op, int tile, int64_t nin, int R
   return g;
 }
 
-// CTAs per SM of star_kernel's real tiles that are sized for it
-// (star_min_ctas), 0 for the others.
-inline int real_resident(const gfd_operator* op, int tile) {
+// CTAs per SM of star_kernel's real tiles up to radius 3, from their registers
+// (bytes: size of a value); 0 for the others.  A residual's figure depends on the
+// radius alone: partials_count() does not know the type.
+inline int real_resident(const gfd_operator* op, int tile, int mode, int bytes) {
   if (op->R > 3) return 0;
-  return tile == TILE_WIDE ? 4 : tile == TILE_48R ? 3 : 0;
+  if (tile == TILE_48R) return 3;
+  if (tile != TILE_WIDE) return 0;
+  if (mode == OP_RESIDUAL) return op->R == 2 ? 3 : 4;
+  if (bytes == 4) return op->R == 3 ? 4 : 5;
+  if (op->R == 1) return mode == OP_APPLY ? 5 : 4;
+  return op->R == 2 && mode == OP_APPLY ? 4 : 3;
 }
 
 template <class S>
@@ -132,12 +138,12 @@ void fill_phases(Phases<S>& P, const double* ph) {
     }
 }
 
-template <class V, int R, int BZ, int TY, int VY, int MODE, int S = kStages>
+template <class V, int R, int BZ, int TY, int VY, int MODE, bool LOW = false, int S = kStages>
 int star_go(const gfd_operator* op, const V* in, V* out, const V* rho, int64_t nin,
             const StarParams<typename vt<V>::S>& base, const LaunchGeom& g, double* partials,
             cudaStream_t s) {
   constexpr size_t smem = star_smem_bytes<BZ, TY, VY, R, S, V, MODE>();
-  auto kern = star_kernel<V, R, BZ, TY, VY, S, MODE>;
+  auto kern = star_kernel<V, R, BZ, TY, VY, S, MODE, LOW>;
   int st = raise_smem_limit(kern, smem, "cudaFuncSetAttribute(star_kernel)");
   if (st) return st;
   StarParams<typename vt<V>::S> p = base;
@@ -187,6 +193,25 @@ constexpr bool has_tile48() {
 // measured slower at every thread shape tried (2110-3570 GB/s): one CTA per
 // SM, or registers short of its 2R + 1 partial sums per row.
 
+// The wide tile of 8-byte values in the form of 2R sums and 128 registers, four
+// CTAs per SM, where the form of 2R + 1 sums leaves room for two or three:
+// complex64 from radius 2 (radius 3: 0.65 to 0.9 of its time in 110 launches of
+// more than two CTAs per SM, 1.0 to 1.1 in 29 smaller ones, which fit the SMs
+// in either form and keep the 2R + 1 sums), and the float64 residual of radius 3
+// (176 registers).  The float64 apply, apply with a potential and Jacobi sweep
+// keep the 2R + 1 sums, three CTAs per SM at radius 3: per CTA and plane both
+// forms take the same time on a full chip (0.25 us), and on grids that do not
+// fill it the form of 2R sums took 9% longer (23 launches).
+template <class V, int R, int MODE>
+constexpr bool wide_low() {
+  return sizeof(V) == 8 && ((vt<V>::NC == 2 && (R == 2 || R == 3)) ||
+                            (vt<V>::NC == 1 && R == 3 && MODE == MODE_RESIDUAL));
+}
+template <class V, int R, int MODE>
+constexpr bool wide_both() {
+  return wide_low<V, R, MODE>() && vt<V>::NC == 2 && R == 3;
+}
+
 template <class V, int R, int MODE>
 int star_wide(const gfd_operator* op, int tile, const V* in, V* out, const V* rho, int64_t nin,
               const StarParams<typename vt<V>::S>& p, const LaunchGeom& g, double* partials,
@@ -201,12 +226,20 @@ int star_wide(const gfd_operator* op, int tile, const V* in, V* out, const V* rh
   }
   if constexpr (vt<V>::NC == 1 && R == 3 && MODE != MODE_RESIDUAL) {
     if (tile == TILE_48R)
-      return star_go<V, R, kTile48Z, 4, 4, MODE>(op, in, out, rho, nin, p, g, partials, s);
+      return star_go<V, R, kTile48Z, 4, 4, MODE, true>(op, in, out, rho, nin, p, g, partials, s);
   }
-  if constexpr (sizeof(V) >= 16 || R > 3)
+  if constexpr (sizeof(V) >= 16 || R > 3) {
     return star_go<V, R, 32, 8, 2, MODE>(op, in, out, rho, nin, p, g, partials, s);
-  else
-    return star_go<V, R, 32, 4, 4, MODE>(op, in, out, rho, nin, p, g, partials, s);
+  } else {
+    if constexpr (wide_low<V, R, MODE>()) {
+      const int64_t ctas = (int64_t)g.grid.x * g.grid.y * g.nxc * nin;
+      if (!wide_both<V, R, MODE>() || ctas > 2 * num_sms())
+        return star_go<V, R, 32, 4, 4, MODE, true>(op, in, out, rho, nin, p, g, partials, s);
+    }
+    if constexpr (!wide_low<V, R, MODE>() || wide_both<V, R, MODE>())
+      return star_go<V, R, 32, 4, 4, MODE>(op, in, out, rho, nin, p, g, partials, s);
+  }
+  return set_error(GFD_EUNSUPPORTED, "star stencil form");  // not reached
 }
 
 template <class V, int MODE>
@@ -760,7 +793,7 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
     }
   }
   LaunchGeom g = star_geom(op, tile, nin, op->R, tuned ? plan.cps : 0,
-                           vt<V>::NC == 1 ? real_resident(op, tile) : 0);
+                           vt<V>::NC == 1 ? real_resident(op, tile, mode, (int)sizeof(V)) : 0);
   p.nxc = g.nxc;
   p.x_chunk = g.x_chunk;
   if (tile == TILE_SPLIT) {
@@ -973,7 +1006,8 @@ inline int64_t partials_count(const gfd_operator* op, int64_t nin) {
   if (op->star) {
     int tile = pick_tile(op);
     TileDims td = tile_dims(tile);
-    LaunchGeom g = star_geom(op, tile, nin, op->R, 0, real_resident(op, tile));
+    LaunchGeom g = star_geom(op, tile, nin, op->R, 0,
+                             real_resident(op, tile, OP_RESIDUAL, 8));
     int gx = (op->n[2] + td.BZ - 1) / td.BZ, gy = (op->n[1] + td.BY - 1) / td.BY;
     return (int64_t)gx * gy * g.nxc * nin;
   }

@@ -294,6 +294,21 @@ def test_fitted_tiles(cuda, N, pbc, n):
         assert rel_err(host(out), ref + v * x) < TOL
 
 
+@pytest.mark.parametrize('nb', [3, 12])
+@pytest.mark.parametrize('n', [1, 2, 3])
+def test_complex64_forms(cuda, nb, n):
+    """complex64 applies past the one-thread-per-point size with fewer and with
+    more than two CTAs per SM, phases on every axis; the FP32 bound of 2e-6."""
+    import torch
+    gd = G.Grid((40, 48, 70), (10.0, 12.0, 17.5), 1)
+    c, o = G.laplace_stencil(gd, -0.5, n)
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((nb, 40, 48, 70)) + 1j * rng.standard_normal((nb, 40, 48, 70))
+    ph = G.bloch_phases(gd, (0.3, -0.2, 0.15))
+    got = gpu_apply(cuda, (gd.N_c, gd.cell_cv, gd.pbc_c), c, o, a, ph, dtype=torch.complex64)
+    assert rel_err(got.astype(complex), K.fd_apply(c, o, gd.pbc_c, a, ph, nthreads=8)) < 2e-6
+
+
 @pytest.mark.parametrize('where', [(3, 5, 7), (0, 0, 0), (19, 59, 46)])
 @pytest.mark.parametrize('value', [float('inf'), float('nan')])
 def test_non_finite_values_stay_within_reach(cuda, where, value):

@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "internal.h"
+#include "march_split.h"
 #include "stencil.cuh"
 #include "stencil_dirs.cuh"
 #include "stencil_flex.cuh"
@@ -66,29 +67,6 @@ int raise_smem_limit(F* kern, size_t bytes, const char* what) {
                     what);
 }
 
-// Axis-0 chunks of a marching launch of `tiles` columns of n0 planes when
-// `resident` CTAs run at a time: the count with the fewest plane steps, a chunk
-// of c planes taking c steps, about 0.7 for each of the 2R planes around it and 3
-// to start, times the waves (at least one).  7 float64 bands of 93 x 113 x 121
-// (196 tiles): 3 chunks, 588 CTAs of 592, 44 us; 4 chunks, the former target of 4
-// CTAs per SM, 50 us.
-inline int best_chunks(int n0, int R, int64_t tiles, int64_t resident) {
-  const int most = std::max(1, n0 / std::max(4, 2 * R));
-  int best = 1;
-  double cost = 0.0;
-  for (int c = 1; c <= most; c++) {
-    const int planes = (n0 + c - 1) / c;
-    const int n = (n0 + planes - 1) / planes;
-    const double waves = std::max(1.0, double(tiles * n) / double(resident));
-    const double t = waves * (planes + 1.4 * R + 3.0);
-    if (cost == 0.0 || t < 0.98 * cost) {
-      cost = t;
-      best = n;
-    }
-  }
-  return best;
-}
-
 struct LaunchGeom {
   dim3 grid;
   int nxc, x_chunk;
@@ -96,7 +74,7 @@ struct LaunchGeom {
 };
 
 // resident: CTAs per SM of the kernel where known (0: aim for march_ctas_per_sm()
-// without counting waves); cps: a launch plan's target.
+// without counting rounds); cps: a launch plan's target.
 inline LaunchGeom star_geom(const gfd_operator* op, int tile, int64_t nin, int R, int cps = 0,
                             int resident = 0) {
   TileDims td = tile_dims(tile);
@@ -108,7 +86,7 @@ inline LaunchGeom star_geom(const gfd_operator* op, int tile, int64_t nin, int R
   int maxc = std::max(1, op->n[0] / std::max(4, 2 * R));
   int nxc = (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles));
   if (cps == 0 && resident > 0)
-    nxc = best_chunks(op->n[0], R, tiles, (int64_t)resident * num_sms());
+    nxc = march_split(op->n[0], R, tiles, resident, num_sms()).chunks;
   g.x_chunk = (op->n[0] + nxc - 1) / nxc;
   g.nxc = (op->n[0] + g.x_chunk - 1) / g.x_chunk;
   g.bands_per_launch = std::max<int64_t>(1, 65535 / g.nxc);
@@ -499,7 +477,7 @@ int march_launches(const gfd_operator* op, int gx, int gy, int64_t nin, int cps,
   const int64_t target = (int64_t)cps * num_sms();  // a launch plan's
   const int nxc =
       cps > 0 ? (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles))
-              : best_chunks(op->n[0], op->R, tiles, (int64_t)resident * num_sms());
+              : march_split(op->n[0], op->R, tiles, resident, num_sms()).chunks;
   p.x_chunk = (op->n[0] + nxc - 1) / nxc;
   p.nxc = (op->n[0] + p.x_chunk - 1) / p.x_chunk;
   const int64_t per_launch = std::max<int64_t>(1, 65535 / p.nxc);
@@ -830,7 +808,19 @@ struct DirGeom {
   int bz, ty, gx, gy, nxc, x_chunk;
   int64_t bands_per_launch;
 };
-inline DirGeom dirs_geom(const gfd_operator* op, int64_t nin) {
+// CTAs per SM of dirs_kernel, from its registers.  As for real_resident, a
+// residual's figure does not depend on the type.
+template <class V>
+int dirs_resident(int R, int mode) {
+  if (mode == OP_RESIDUAL) return 2;
+  if (sizeof(V) == 16) return R == 1 ? 3 : 2;
+  if (sizeof(V) == 4) return R <= 3 ? 4 : 3;
+  if (vt<V>::NC == 2) return R <= 2 ? 3 : 2;
+  if (mode != OP_APPLY) return R == 1 ? 3 : 2;
+  return R == 1 ? 4 : R <= 3 ? 3 : 2;
+}
+
+inline DirGeom dirs_geom(const gfd_operator* op, int resident, int64_t nin) {
   const int R = op->mp;
   DirGeom g;
   g.gx = (op->n[2] + kDirBZ - 1) / kDirBZ;
@@ -847,7 +837,7 @@ inline DirGeom dirs_geom(const gfd_operator* op, int64_t nin) {
   g.ty = (rows + kDirVY - 1) / kDirVY;
   g.gy = (op->n[1] + g.ty * kDirVY - 1) / (g.ty * kDirVY);
   const int64_t tiles = (int64_t)g.gx * g.gy * std::max<int64_t>(nin, 1);
-  const int nxc = best_chunks(op->n[0], R, tiles, 2LL * num_sms());
+  const int nxc = march_split(op->n[0], R, tiles, resident, num_sms()).chunks;
   g.x_chunk = (op->n[0] + nxc - 1) / nxc;
   g.nxc = (op->n[0] + g.x_chunk - 1) / g.x_chunk;
   g.bands_per_launch = std::max<int64_t>(1, 65535 / g.nxc);
@@ -918,7 +908,7 @@ template <class V, int MODE>
 int dirs_dispatch(const gfd_operator* op, int mode, const V* in, V* out, const V* rho,
                   int64_t nin, const double* phase_cd, double w, double* partials,
                   cudaStream_t s) {
-  const DirGeom g = dirs_geom(op, nin);
+  const DirGeom g = dirs_geom(op, dirs_resident<V>(op->mp, mode), nin);
   DirParams<typename vt<V>::S> p;
   dirs_params(op, mode, w, phase_cd, g, p);
   switch (op->mp) {
@@ -1012,7 +1002,7 @@ inline int64_t partials_count(const gfd_operator* op, int64_t nin) {
     return (int64_t)gx * gy * g.nxc * nin;
   }
   if (dirs_eligible(op, OP_RESIDUAL)) {
-    const DirGeom g = dirs_geom(op, nin);
+    const DirGeom g = dirs_geom(op, dirs_resident<double>(op->mp, OP_RESIDUAL), nin);
     return (int64_t)g.gx * g.gy * g.nxc * nin;
   }
   const int BZ = 32, BY = 8;

@@ -273,3 +273,45 @@ def test_coefficient_limit_holds_for_every_stencil_class():
                                      ctypes.addressof(buf) + 4096, 1, None, None)
     assert st == _lib.GFD_EUNSUPPORTED and 'coefficients' in _lib.last_error()
     assert _lib.lib.gfd_operator_destroy(h) == 0
+
+
+def test_march_split_counts_whole_rounds(tmp_path):
+    """The axis-0 split of the marching kernels (march_split.h, built with the
+    host compiler): a launch a little past a round of CTAs is cut further, one
+    that fits is not, and the split is the best of its rule for all sizes."""
+    import subprocess
+    src = tmp_path / 'split.cpp'
+    src.write_text('#include "march_split.h"\n'
+                   'extern "C" int split(int n0, int R, long long tiles, int res, int sms,\n'
+                   '                     double* steps) {\n'
+                   '  auto s = gfd::march_split(n0, R, tiles, res, sms);\n'
+                   '  *steps = s.steps;\n  return s.chunks;\n}\n')
+    lib = tmp_path / 'split.so'
+    subprocess.run(['g++', '-std=c++17', '-O1', '-shared', '-fPIC', '-I',
+                    os.path.join(ROOT, 'gpaw_b200', 'csrc'), str(src), '-o', str(lib)], check=True)
+    f = ctypes.CDLL(str(lib)).split
+
+    def split(n0, R, tiles, res, sms=148):
+        steps = ctypes.c_double()
+        return f(n0, R, ctypes.c_longlong(tiles), res, sms, ctypes.byref(steps)), steps.value
+
+    def rounds(ctas, res, sms=148):
+        whole, rest = divmod(ctas, res * sms)
+        return whole + (0.5 + 0.5 * -(-rest // sms) / res if rest else 0.0)
+
+    assert split(66, 3, 300, 2)[0] > 1       # 300 CTAs on 296 slots
+    assert split(66, 3, 296, 2)[0] == 1
+    assert split(80, 3, 160, 2) == (3, 66.0)  # 480 CTAs in two rounds of 33 steps
+    assert split(1, 3, 5, 2) == (1, 0.75 * 7)
+    rng = np.random.default_rng(1)
+    for _ in range(300):
+        n0, R, res = int(rng.integers(1, 200)), int(rng.integers(1, 7)), int(rng.integers(1, 6))
+        tiles = int(2 ** rng.uniform(0, 13))
+        chunks, steps = split(n0, R, tiles, res)
+        planes = -(-n0 // chunks)
+        assert chunks == -(-n0 // planes) and (chunks == 1 or planes >= min(n0, max(4, 2 * R)))
+        assert abs(steps - rounds(tiles * chunks, res) * (planes + 2 * R)) < 1e-9
+        limit = 12 * res * 148 // tiles + 1
+        for c in range(1, min(max(1, n0 // max(4, 2 * R)), limit) + 1):
+            p = -(-n0 // c)
+            assert steps <= rounds(tiles * -(-n0 // p), res) * (p + 2 * R) + 1e-9

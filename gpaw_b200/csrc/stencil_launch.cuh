@@ -887,11 +887,11 @@ void dirs_params(const gfd_operator* op, int mode, double w, const double* phase
           p.fix_yz = 1;
 }
 
-template <class V, int R, int MODE>
-int dirs_go(const gfd_operator* op, const V* in, V* out, const V* rho, int64_t nin,
-            DirParams<typename vt<V>::S>& p, const DirGeom& g, double* partials,
-            cudaStream_t s) {
-  auto kern = dirs_kernel<V, R, kDirVY, kDirNT, 2, kDirBZ, kDirCPT, kDirStages, MODE>;
+template <class V, int R, int MODE, bool FULL>
+int dirs_launch(const gfd_operator* op, const V* in, V* out, const V* rho, int64_t nin,
+                DirParams<typename vt<V>::S>& p, const DirGeom& g, double* partials,
+                cudaStream_t s) {
+  auto kern = dirs_kernel<V, R, kDirVY, kDirNT, 2, kDirBZ, kDirCPT, kDirStages, MODE, FULL>;
   const size_t smem = dirs_smem_bytes<V, R, kDirVY, kDirNT, kDirBZ, kDirStages>(g.ty);
   int st = raise_smem_limit(kern, smem, "cudaFuncSetAttribute(dirs_kernel)");
   if (st) return st;
@@ -902,6 +902,16 @@ int dirs_go(const gfd_operator* op, const V* in, V* out, const V* rho, int64_t n
              out + b0 * p.band, rho ? rho + b0 * p.band : nullptr, p);
   }
   return check_launch("dirs_kernel");
+}
+
+template <class V, int R, int MODE>
+int dirs_go(const gfd_operator* op, const V* in, V* out, const V* rho, int64_t nin,
+            DirParams<typename vt<V>::S>& p, const DirGeom& g, double* partials,
+            cudaStream_t s) {
+  if constexpr (sizeof(V) == 16 || (sizeof(V) == 8 && vt<V>::NC == 1)) {
+    if (p.xmask == 7u) return dirs_launch<V, R, MODE, true>(op, in, out, rho, nin, p, g, partials, s);
+  }
+  return dirs_launch<V, R, MODE, false>(op, in, out, rho, nin, p, g, partials, s);
 }
 
 template <class V, int MODE>

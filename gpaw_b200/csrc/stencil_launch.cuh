@@ -107,6 +107,20 @@ inline int real_resident(const gfd_operator* op, int tile, int mode, int bytes) 
   return op->R == 2 && mode == OP_APPLY ? 4 : 3;
 }
 
+// The real 48-column tile where its launch takes less time than the wide one's:
+// a CTA of its full SM steps once in 1.18 us (float32 0.80) against 0.76 (0.68),
+// fitted as in march_split.h.
+inline bool tile48r_pays(const gfd_operator* op, int mode, int bytes, int64_t nin) {
+  auto steps = [&](int tile) {
+    const TileDims td = tile_dims(tile);
+    const int64_t tiles =
+        (int64_t)((op->n[1] + td.BY - 1) / td.BY) * ((op->n[2] + td.BZ - 1) / td.BZ) * nin;
+    return march_split(op->n[0], op->R, tiles, real_resident(op, tile, mode, bytes), num_sms())
+        .steps;
+  };
+  return steps(TILE_48R) * (bytes == 4 ? 0.80 : 1.18) < steps(TILE_WIDE) * (bytes == 4 ? 0.68 : 0.76);
+}
+
 template <class S>
 void fill_phases(Phases<S>& P, const double* ph) {
   for (int c = 0; c < 3; c++)
@@ -726,7 +740,7 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
     tile = c128_tile(op, mode, tile);
   // real bands: 16 of 47^3 17.7 us against 21.1 us (two 32-column tiles)
   const bool t48rok = vt<V>::NC == 1 && mode != OP_RESIDUAL && tile48r_eligible(op);
-  if (t48rok && tile == TILE_WIDE) tile = TILE_48R;
+  if (t48rok && tile == TILE_WIDE && tile48r_pays(op, mode, (int)sizeof(V), nin)) tile = TILE_48R;
   if (tuned) {
     if (plan.tile == TILE_PAIR)
       tile = pairok ? TILE_PAIR : tile;

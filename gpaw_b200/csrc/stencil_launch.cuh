@@ -502,11 +502,31 @@ int march_launches(const gfd_operator* op, int gx, int gy, int64_t nin, int cps,
   return GFD_OK;
 }
 
-// The tile with the least work per plane, threads that run plus a quarter per
-// staged cell; a narrower tile has to save 6% (its rows start more staged
-// segments).  Measured for 108^3 R = 3: (36, 6) 692 us, (36, 7) 725, (54, 4)
-// 796; 90 x 100: (50, 5) 430, (26, 9) and (34, 7) slower; 96^2: (32, 8) 928,
-// (48, 5) 989, (48, 4) 1006.
+// Time of one plane step of a CTA with its SM full, in microseconds, and the
+// CTAs that an SM holds (registers).  Fitted to 22000 launches of the four
+// kernels (grids of 24 to 144 points a side, 1 to 64 bands, every axis-0 split,
+// zero and periodic boundaries; 7 to 10% rms) with march_split.h's rounds.  A
+// potential adds 11% to each.
+struct StepCost {
+  double us;
+  int resident;
+};
+inline double flex_step_us(const FlexTile& t, int R) {
+  // a staged row costs as much as 20 staged cells
+  return 0.15 + 0.00073 * flex_cells(t, R) + 0.0152 * (t.ty * kFlexVY + 2 * R);
+}
+inline StepCost c128_fixed_cost(int tile, int R) {
+  const double us = tile == TILE_48 ? 0.45 + 0.11 * R : 0.28 + 0.184 * R;
+  const int resident = tile == TILE_48 ? 2 : 3;
+  if (R > 1) return {us, resident};
+  return {us * (resident + 1) / resident, resident + 1};
+}
+// Bloch phases of axes 1 and 2 cost the pair kernel 63%, the others 39 to 47%.
+inline StepCost pair_cost(bool phases) { return {phases ? 1.30 : 1.11, 3}; }
+
+// The tile with the least time per plane.  Measured for 108^3 R = 3, 64 bands:
+// (36, 6) 692 us, (36, 7) 725, (54, 4) 796; 90 x 100: (50, 5) 430, (26, 9) and
+// (34, 7) slower; 96^2: (32, 8) 928, (48, 5) 989, (48, 4) 1006.
 inline FlexTile flex_tile(const gfd_operator* op, int mode) {
   const int n1 = op->n[1], n2 = op->n[2], R = op->R;
   // two CTAs per SM
@@ -520,8 +540,6 @@ inline FlexTile flex_tile(const gfd_operator* op, int mode) {
     if (t.bz == last) continue;
     last = t.bz;
     if (t.bz < 16 && cost > 0.0) break;
-    double c_bz = 0.0;
-    int ty_bz = 1;
     const int most = std::min(kFlexNT / t.bz, (n1 + kFlexVY - 1) / kFlexVY);
     for (t.ty = 1; t.ty <= most; t.ty++) {
       if (flex_cells(t, R) > kFlexCPT * kFlexNT ||
@@ -529,41 +547,61 @@ inline FlexTile flex_tile(const gfd_operator* op, int mode) {
         break;
       const double tiles = double((n2 + t.bz - 1) / t.bz) *
                            ((n1 + t.ty * kFlexVY - 1) / (t.ty * kFlexVY));
-      const double c = tiles * (t.bz * t.ty + 0.25 * flex_cells(t, R));
-      if (c_bz == 0.0 || c < c_bz) {
-        c_bz = c;
-        ty_bz = t.ty;
+      const double c = tiles * flex_step_us(t, R);
+      if (cost == 0.0 || c < cost) {
+        cost = c;
+        best = t;
       }
-    }
-    if (c_bz > 0.0 && (cost == 0.0 || c_bz < 0.94 * cost)) {
-      cost = c_bz;
-      best = {t.bz, ty_bz};
     }
   }
   return best;
+}
+inline PairTile pair_tile(const gfd_operator* op) {
+  // 32 columns by 12 rows; fewer where the grid is smaller
+  const int gx = (op->n[2] + kPairBZ - 1) / kPairBZ;
+  PairTile t;
+  t.bz = ((op->n[2] + gx - 1) / gx + 1) / 2 * 2;
+  t.ty = std::min(4, (op->n[1] + kPairVY - 1) / kPairVY);
+  return t;
 }
 // Points of the padded plane of a tile.
 inline long long padded(int n1, int n2, int by, int bz) {
   return (long long)((n1 + by - 1) / by * by) * ((n2 + bz - 1) / bz * bz);
 }
 // Built-in choice for complex128 up to radius 3 past the one-thread-per-point
-// size (`fixed`: the fixed-side tile that would be taken).  Applies: the pair
-// kernel at radius 3 where its 32 x 12 tiles pad either axis by 3% at most
-// (4424 against 3949 GB/s on 96^3, 4169 against 3908 on 128 x 120 x 128, but 3733
-// against 3983 on 64^3), else the flex kernel (64^3 3983 against 3691 for the
-// 32 x 8 tile, 90 x 100 3598 against 2867; radius 1 5998 against 5248, radius
-// 2 4287 against 4010).  The other modes: flex where the fixed tile pads the
-// plane 8% more (potential 90 x 100: 3237 against 2521, but 3113 against 3639
-// on 96^2 for the 48 x 8 tile; Jacobi 104^2 2623 against 1929, but 2619
-// against 2685 on 96^2).
-inline int c128_tile(const gfd_operator* op, int mode, int fixed) {
+// size (`fixed`: the fixed-side tile that would be taken; phases: Bloch phases on
+// axes 1 or 2).
+// Applies: the kernel whose launch takes the least time by the costs above, the
+// fixed-side tile unless another saves 3%.  498 launches, one B200, times
+// against the fixed-side tiles and four CTAs per SM for all: 0.87 in the
+// geometric mean, 1.00 at the 90th percentile; with flex or pair tiles for every
+// grid, whatever the bands, 0.98 and 1.23.
+// Jacobi and residual sweeps: flex where the fixed tile pads the plane 8% more
+// (Jacobi 104^2 2623 GB/s against 1929, but 2619 against 2685 on 96^2).
+inline int c128_tile(const gfd_operator* op, int mode, int fixed, int64_t nin, bool phases) {
   const int n1 = op->n[1], n2 = op->n[2];
-  if (mode == OP_APPLY && op->R == kPairR) {
-    const int gx = (n2 + kPairBZ - 1) / kPairBZ, by = 4 * kPairVY, gy = (n1 + by - 1) / by;
-    if (gx * kPairBZ - n2 <= n2 / 32 && gy * by - n1 <= n1 / 32) return TILE_PAIR;
-  }
-  if (mode == OP_APPLY) return TILE_FLEX;
   const FlexTile f = flex_tile(op, mode);
+  if (mode == OP_APPLY || mode == OP_POTENTIAL) {
+    int tile = fixed;
+    double cost = 0.0;
+    auto consider = [&](int cand, int by, int bz, const StepCost& c) {
+      const int64_t tiles = (int64_t)((n1 + by - 1) / by) * ((n2 + bz - 1) / bz) * nin;
+      const double t = march_split(op->n[0], op->R, tiles, c.resident, num_sms()).steps * c.us;
+      if (cost == 0.0 || t < cost) {
+        tile = cand;
+        cost = cost == 0.0 ? 0.97 * t : t;
+      }
+    };
+    const TileDims td = tile_dims(fixed);
+    consider(fixed, td.BY, td.BZ, c128_fixed_cost(fixed, op->R));
+    consider(TILE_FLEX, f.ty * kFlexVY, f.bz, {flex_step_us(f, op->R), 2});
+    if (mode == OP_APPLY && op->R == kPairR) {
+      const PairTile t = pair_tile(op);
+      consider(TILE_PAIR, t.ty * kPairVY, t.bz, pair_cost(phases));
+    }
+    if (fixed == TILE_48) consider(TILE_SHORT, 8, kShortTileZ, c128_fixed_cost(TILE_SHORT, op->R));
+    return tile;
+  }
   const TileDims td = tile_dims(fixed);
   return padded(n1, n2, td.BY, td.BZ) * 100 > padded(n1, n2, f.ty * kFlexVY, f.bz) * 108
              ? TILE_FLEX
@@ -572,11 +610,8 @@ inline int c128_tile(const gfd_operator* op, int mode, int fixed) {
 
 inline int pair_launch(const gfd_operator* op, const cplx<double>* in, cplx<double>* out,
                        int64_t nin, StarParams<double> p, int cps, cudaStream_t s) {
-  // 32 columns by 12 rows; fewer where the grid is smaller
-  const int gx = (op->n[2] + kPairBZ - 1) / kPairBZ;
-  PairTile t;
-  t.bz = ((op->n[2] + gx - 1) / gx + 1) / 2 * 2;
-  t.ty = std::min(4, (op->n[1] + kPairVY - 1) / kPairVY);
+  const PairTile t = pair_tile(op);
+  const int gx = (op->n[2] + t.bz - 1) / t.bz;
   const int gy = (op->n[1] + t.ty * kPairVY - 1) / (t.ty * kPairVY);
   const size_t smem = pair_smem_bytes(t.ty);
   int st = raise_smem_limit(star_pair_kernel, smem, "cudaFuncSetAttribute(star_pair_kernel)");
@@ -737,7 +772,7 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
   const bool flexok = sizeof(V) >= 16 && op->R <= kFlexR;
   const bool pairok = sizeof(V) >= 16 && op->R == kPairR && mode == OP_APPLY;
   if (flexok && (tile == TILE_WIDE || tile == TILE_SHORT || tile == TILE_48))
-    tile = c128_tile(op, mode, tile);
+    tile = c128_tile(op, mode, tile, nin, p.fix_yz != 0);
   // real bands: 16 of 47^3 17.7 us against 21.1 us (two 32-column tiles)
   const bool t48rok = vt<V>::NC == 1 && mode != OP_RESIDUAL && tile48r_eligible(op);
   if (t48rok && tile == TILE_WIDE && tile48r_pays(op, mode, (int)sizeof(V), nin)) tile = TILE_48R;
@@ -784,8 +819,11 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
       return flex_dispatch<MODE_APPLY>(op, mode, vin, vout, nullptr, nin, p, cps, s);
     }
   }
-  LaunchGeom g = star_geom(op, tile, nin, op->R, tuned ? plan.cps : 0,
-                           vt<V>::NC == 1 ? real_resident(op, tile, mode, (int)sizeof(V)) : 0);
+  int resident = 0;
+  if (vt<V>::NC == 1) resident = real_resident(op, tile, mode, (int)sizeof(V));
+  if (flexok && (tile == TILE_SHORT || tile == TILE_48))
+    resident = c128_fixed_cost(tile, op->R).resident;
+  LaunchGeom g = star_geom(op, tile, nin, op->R, tuned ? plan.cps : 0, resident);
   p.nxc = g.nxc;
   p.x_chunk = g.x_chunk;
   if (tile == TILE_SPLIT) {

@@ -513,7 +513,7 @@ struct StepCost {
 };
 inline double flex_step_us(const FlexTile& t, int R) {
   // a staged row costs as much as 20 staged cells
-  return 0.15 + 0.00073 * flex_cells(t, R) + 0.0152 * (t.ty * kFlexVY + 2 * R);
+  return 0.155 + 0.00075 * flex_cells(t, R) + 0.0157 * (t.ty * kFlexVY + 2 * R);
 }
 inline StepCost c128_fixed_cost(int tile, int R) {
   const double us = tile == TILE_48 ? 0.45 + 0.11 * R : 0.28 + 0.184 * R;
@@ -522,15 +522,16 @@ inline StepCost c128_fixed_cost(int tile, int R) {
   return {us * (resident + 1) / resident, resident + 1};
 }
 // Bloch phases of axes 1 and 2 cost the pair kernel 63%, the others 39 to 47%.
-inline StepCost pair_cost(bool phases) { return {phases ? 1.30 : 1.11, 3}; }
+inline StepCost pair_cost(bool phases) { return {phases ? 1.38 : 1.18, 3}; }
 
 // The tile with the least time per plane.  Measured for 108^3 R = 3, 64 bands:
 // (36, 6) 692 us, (36, 7) 725, (54, 4) 796; 90 x 100: (50, 5) 430, (26, 9) and
 // (34, 7) slower; 96^2: (32, 8) 928, (48, 5) 989, (48, 4) 1006.
 inline FlexTile flex_tile(const gfd_operator* op, int mode) {
   const int n1 = op->n[1], n2 = op->n[2], R = op->R;
-  // two CTAs per SM
-  const size_t most_smem = 112 * 1024 - (mode == OP_APPLY ? 0 : mode == OP_POTENTIAL ? 16 : 32) * 1024;
+  // Two CTAs in 196 KB, so that 60 KB stay with L1: tiles past that took 18 to
+  // 24% longer than their cost (20 launches).
+  const size_t most_smem = 97 * 1024 - (mode == OP_APPLY ? 0 : mode == OP_POTENTIAL ? 16 : 32) * 1024;
   FlexTile best = {std::min(n2, 8), 1};
   double cost = 0.0;
   int last = 0;

@@ -443,6 +443,18 @@ star_kernel(const V* __restrict__ in, V* __restrict__ out, const V* __restrict__
   }
 }
 
+// Distances per axis that star_point_at loads together (a divisor of 2R): all of
+// them in flight need 2R values of each axis in registers, which 16-byte values
+// and complex64 past radius 4 pay for with warps.  490 launches up to 300000
+// points, against one neighbour after the other: complex128 radius 6 0.83 to
+// 0.88 of the time with two (all twelve 1.25 to 1.7), radius 4 0.78 with four
+// (1.0), radius 2 0.89 with two (0.96); complex64 radius 5 0.64 with five (0.89).
+template <class V, int R>
+constexpr int direct_group() {
+  if (sizeof(V) >= 16) return R >= 5 ? 2 : R;
+  if (vt<V>::NC == 2 && R >= 5) return R;
+  return 2 * R;
+}
 // ---------------------------------------------------------------------------
 // Direct star stencil: one thread per point, neighbours read through the L1
 // cache.  For small grids (the coarse multigrid levels) the marching kernel
@@ -467,27 +479,36 @@ __device__ __forceinline__ V star_point_at(const V* __restrict__ base, const V* 
   const int pl = p.n1 * p.n2, row = i0 * pl + i1 * p.n2, ownr = int(rem);
   V src = vzero<V>();
   if constexpr (MODE == MODE_JACOBI || MODE == MODE_RESIDUAL) src = LD::ld(rho_b + rem);
-  // All loads first: left to itself the compiler keeps to 32 registers and
-  // waits for one neighbour after the other.
-  V v[3][2 * R];
+  // Loads of G distances on each axis together: left to itself the compiler
+  // keeps to 32 registers and waits for one neighbour after the other.
+  constexpr int G = direct_group<V, R>();
+  auto group = [&](int k0) {
+    V v[3][G];
 #pragma unroll
-  for (int k = 0; k < 2 * R; k++) {
-    const int d = k < R ? k - R : k - R + 1;
-    int sd;
-    bool ok;
-    int j = map_axis(i0 + d, p.n0, p.per0, sd, ok);
-    v[0][k] = side_phase(p.P, 0, sd, value_or_zero(ok, LD::ld(base + (j * pl + (ownr - i0 * pl)))));
-    j = map_axis(i1 + d, p.n1, p.per1, sd, ok);
-    v[1][k] = side_phase(p.P, 1, sd, value_or_zero(ok, LD::ld(base + (i0 * pl + j * p.n2 + i2))));
-    j = map_axis(i2 + d, p.n2, p.per2, sd, ok);
-    v[2][k] = side_phase(p.P, 2, sd, value_or_zero(ok, LD::ld(base + (row + j))));
-  }
+    for (int k = 0; k < G; k++) {
+      const int d = k0 + k < R ? k0 + k - R : k0 + k - R + 1;
+      int sd;
+      bool ok;
+      int j = map_axis(i0 + d, p.n0, p.per0, sd, ok);
+      v[0][k] = side_phase(p.P, 0, sd, value_or_zero(ok, LD::ld(base + (j * pl + (ownr - i0 * pl)))));
+      j = map_axis(i1 + d, p.n1, p.per1, sd, ok);
+      v[1][k] = side_phase(p.P, 1, sd, value_or_zero(ok, LD::ld(base + (i0 * pl + j * p.n2 + i2))));
+      j = map_axis(i2 + d, p.n2, p.per2, sd, ok);
+      v[2][k] = side_phase(p.P, 2, sd, value_or_zero(ok, LD::ld(base + (row + j))));
+    }
 #pragma unroll
-  for (int k = 0; k < 2 * R; k++) {
-    const int d = k < R ? k - R : k - R + 1;
-    madd(s, p.cx[kMaxR + d], v[0][k]);
-    madd(s, p.cy[kMaxR + d], v[1][k]);
-    madd(s, p.cz[kMaxR + d], v[2][k]);
+    for (int k = 0; k < G; k++) {
+      const int d = k0 + k < R ? k0 + k - R : k0 + k - R + 1;
+      madd(s, p.cx[kMaxR + d], v[0][k]);
+      madd(s, p.cy[kMaxR + d], v[1][k]);
+      madd(s, p.cz[kMaxR + d], v[2][k]);
+    }
+  };
+  if constexpr (G == 2 * R) {
+    group(0);
+  } else {
+#pragma unroll 1
+    for (int k0 = 0; k0 < 2 * R; k0 += G) group(k0);
   }
   if constexpr (MODE == MODE_JACOBI) return vmul(p.wc, vsub(src, s));
   else if constexpr (MODE == MODE_RESIDUAL) return vsub(s, src);

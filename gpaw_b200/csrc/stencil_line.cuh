@@ -18,11 +18,8 @@
 
 namespace gfd {
 
-// Values loaded at a time: 8-byte ones and smaller 8, complex128 4.
-template <class V>
-constexpr int line_block() {
-  return 4;
-}
+// Values loaded at a time (8: 171 us against 157, 200 against 180).
+constexpr int kLineBlock = 4;
 
 template <class S>
 struct LineParams {
@@ -46,7 +43,7 @@ __global__ void __launch_bounds__(256)
 line_march_kernel(const V* __restrict__ in, V* __restrict__ out,
                   const LineParams<typename vt<V>::S> p) {
   pdl_enter();
-  constexpr int B = line_block<V>(), W = B + 2 * R;
+  constexpr int B = kLineBlock, W = B + 2 * R;
   const long long i = blockIdx.x * 256LL + threadIdx.x;
   if (i >= p.inner) return;
   const int c = blockIdx.y;
@@ -60,7 +57,8 @@ line_march_kernel(const V* __restrict__ in, V* __restrict__ out,
       if (j < 0) return vzero<V>();
       V v = ldro(a + j * p.inner);
       if constexpr (vt<V>::NC == 2) {
-        if (side >= 0) v = phase_mul(p.ph[side], v);
+        // not p.ph[side]: an index of the parameters copies them to local memory
+        if (side >= 0) v = phase_mul(side == 1 ? p.ph[1] : p.ph[0], v);
       }
       return v;
     };

@@ -294,11 +294,12 @@ def test_fitted_tiles(cuda, N, pbc, n):
         assert rel_err(host(out), ref + v * x) < TOL
 
 
-@pytest.mark.parametrize('nb', [3, 12])
-@pytest.mark.parametrize('n', [1, 2, 3])
+@pytest.mark.parametrize('nb', [1, 3, 12])
+@pytest.mark.parametrize('n', [1, 2, 3, 4, 5, 6])
 def test_complex64_forms(cuda, nb, n):
-    """complex64 applies past the one-thread-per-point size with fewer and with
-    more than two CTAs per SM, phases on every axis; the FP32 bound of 2e-6."""
+    """complex64 applies of one thread per point, and past that size with fewer
+    and with more than two CTAs per SM; phases on every axis, the FP32 bound of
+    2e-6."""
     import torch
     gd = G.Grid((40, 48, 70), (10.0, 12.0, 17.5), 1)
     c, o = G.laplace_stencil(gd, -0.5, n)

@@ -675,18 +675,19 @@ int line_go(const gfd_operator* op, int axis, const V* in, V* out, int64_t nin,
   }
   p.inner = axis == 0 ? (long long)n1 * n2 : n2;
   p.outer = axis == 0 ? nin : nin * n0;
-  // Whole lines per thread once that fills the chip a few times over; chunks
-  // of at least 4 (2R) outputs, whose 2R extra values come from L2, below.
-  const long long threads = p.inner * p.outer, want = 4LL * 2048 * num_sms();
-  const int maxc = std::max(1, p.n / (8 * R));
-  p.nch = (int)std::min<long long>(maxc, std::max<long long>(1, want / std::max(1LL, threads)));
+  // Whole lines per thread once that fills the chip a few times over; below,
+  // chunks of at least 4 (2R) outputs, whose 2R extra values come from L2, and
+  // down to 2R outputs where the chip would not be full once.
+  const long long threads = p.inner * p.outer, fill = 2048LL * num_sms();
+  const int maxc = std::max(1, p.n / (8 * R)), most = std::max(1, p.n / std::max(4, 2 * R));
+  p.nch = (int)std::min<long long>(maxc, std::max<long long>(1, 4 * fill / threads));
+  if (threads * p.nch < fill)
+    p.nch = (int)std::min<long long>(most, (fill + threads - 1) / threads);
   p.chunk = (p.n + p.nch - 1) / p.nch;
   p.nch = (p.n + p.chunk - 1) / p.chunk;
-  const int nt = p.inner >= 256 ? 256 : (int)((p.inner + 31) / 32 * 32);
-  const long long gx = (p.inner + nt - 1) / nt;
-  launch_k(line_march_kernel<V, R>,
-           dim3((unsigned)gx, (unsigned)p.nch, (unsigned)std::min<long long>(p.outer, 65535)), nt,
-           0, s, in, out, p);
+  const long long blocks = (threads + 255) / 256;
+  if (blocks > 0x7fffffffLL) return set_error(GFD_EUNSUPPORTED, "too many lines");
+  launch_k(line_march_kernel<V, R>, dim3((unsigned)blocks, (unsigned)p.nch), 256, 0, s, in, out, p);
   return check_launch("line_march_kernel");
 }
 

@@ -44,41 +44,43 @@ line_march_kernel(const V* __restrict__ in, V* __restrict__ out,
                   const LineParams<typename vt<V>::S> p) {
   pdl_enter();
   constexpr int B = kLineBlock, W = B + 2 * R;
-  const long long i = blockIdx.x * 256LL + threadIdx.x;
-  if (i >= p.inner) return;
+  const long long g = blockIdx.x * 256LL + threadIdx.x, lines = p.inner * p.outer;
+  if (g >= lines) return;
+  // Lanes run over the lines as they lie in memory, past the end of one step of
+  // the axis into the next: no lane idles where p.inner is not a multiple of 32.
+  const long long o = lines <= 0x7fffffff ? int(g) / int(p.inner) : g / p.inner;
   const int c = blockIdx.y;
   const int x0 = c * p.chunk, x1 = min(p.n, x0 + p.chunk);
-  for (long long o = blockIdx.z; o < p.outer; o += gridDim.z) {
-    const V* a = in + o * p.n * p.inner + i;
-    V* b = out + o * p.n * p.inner + i;
-    auto load = [&](int u) -> V {
-      int side;
-      const int j = wrap_plane(u, p.n, p.per, side);
-      if (j < 0) return vzero<V>();
-      V v = ldro(a + j * p.inner);
-      if constexpr (vt<V>::NC == 2) {
-        // not p.ph[side]: an index of the parameters copies them to local memory
-        if (side >= 0) v = phase_mul(side == 1 ? p.ph[1] : p.ph[0], v);
-      }
-      return v;
-    };
-    V win[W];
-#pragma unroll
-    for (int k = 0; k < 2 * R; k++) win[k] = load(x0 - R + k);
-    for (int x = x0; x < x1; x += B) {
-#pragma unroll
-      for (int k = 0; k < B; k++) win[2 * R + k] = x + R + k < x1 + R ? load(x + R + k) : vzero<V>();
-#pragma unroll
-      for (int j = 0; j < B; j++) {
-        V s = centre(p, win[j + R]);
-#pragma unroll
-        for (int k = -R; k <= R; k++)
-          if (k != 0) madd(s, p.w[kMaxR + k], win[j + R + k]);
-        if (x + j < x1) stcs(b + (x + j) * p.inner, s);
-      }
-#pragma unroll
-      for (int k = 0; k < 2 * R; k++) win[k] = win[k + B];
+  const long long at = o * (p.n - 1) * p.inner + g;  // o whole lines and g - o inner
+  const V* a = in + at;
+  V* b = out + at;
+  auto load = [&](int u) -> V {
+    int side;
+    const int j = wrap_plane(u, p.n, p.per, side);
+    if (j < 0) return vzero<V>();
+    V v = ldro(a + j * p.inner);
+    if constexpr (vt<V>::NC == 2) {
+      // not p.ph[side]: an index of the parameters copies them to local memory
+      if (side >= 0) v = phase_mul(side == 1 ? p.ph[1] : p.ph[0], v);
     }
+    return v;
+  };
+  V win[W];
+#pragma unroll
+  for (int k = 0; k < 2 * R; k++) win[k] = load(x0 - R + k);
+  for (int x = x0; x < x1; x += B) {
+#pragma unroll
+    for (int k = 0; k < B; k++) win[2 * R + k] = x + R + k < x1 + R ? load(x + R + k) : vzero<V>();
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+      V s = centre(p, win[j + R]);
+#pragma unroll
+      for (int k = -R; k <= R; k++)
+        if (k != 0) madd(s, p.w[kMaxR + k], win[j + R + k]);
+      if (x + j < x1) stcs(b + (x + j) * p.inner, s);
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * R; k++) win[k] = win[k + B];
   }
 }
 

@@ -743,9 +743,8 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
     return direct_dispatch<V, MODE_APPLY>(op, vin, vout, nullptr, p, nin, s);
   }
   if (mode == OP_APPLY) {
-    const int axis = line_axis(op);
-    if (axis >= 0 && (axis < 2 || op->n[2] <= 1024))
-      return line_dispatch<V>(op, axis, vin, vout, nin, phase_cd, s);
+    const int axis = line_apply_axis(op, (int)sizeof(V), nin);
+    if (axis >= 0) return line_dispatch<V>(op, axis, vin, vout, nin, phase_cd, s);
   }
   if constexpr (std::is_same_v<V, cplx<double>>) {
     if (!tuned && mode == OP_APPLY && tma_eligible(op, in)) {

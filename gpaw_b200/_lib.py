@@ -47,9 +47,10 @@ class TunePlan(ctypes.Structure):
     """gfd_tune_plan: form 0 one thread per point / 1 marching kernel, the
     marching tile (0: 32 columns, 1: 16, 2: 8, 3: 32 columns by 8 rows, 4: complex
     bands with the real and imaginary parts on lane pairs, 5: the same for
-    complex128 on full rows staged by TMA, 6: complex128, 48 columns by 8
-    rows), the
-    axis-0 split target in CTAs per SM and the measured microseconds per
+    complex128 on full rows staged by TMA, 6: complex bands, 48 columns by 8
+    rows, 7: complex128 apply of radius 3, two columns per lane pair, 8: real
+    bands of radius 3, 48 columns by 16 rows, 9: complex128 up to radius 3, tile
+    sides that fit the grid), the axis-0 split target in CTAs per SM and the measured microseconds per
     launch."""
     _fields_ = [('form', ctypes.c_int), ('tile', ctypes.c_int), ('ctas_per_sm', ctypes.c_int),
                 ('us', ctypes.c_double)]

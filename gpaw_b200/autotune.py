@@ -6,8 +6,9 @@ per point or the marching kernel), the marching tile and the axis-0 split.
 Without a tuned plan it uses built-in rules; tune_operator / tune_transformer
 time every candidate on the GPU and cache the fastest in the library, where
 every later launch with the same key finds it.  Plans change times; the
-results of the marching candidates are bit-identical, the one-thread-per-point
-form sums a stencil's terms in another order (rounding-level differences).
+results of most tiles are bit-identical, the lane-pair and column-pair tiles and
+the one-thread-per-point form sum a stencil's terms in other orders
+(rounding-level differences).
 
     from gpaw_b200 import autotune
     autotune.tune_operator(lap, nbands=512, phase_cd=phase_cd)

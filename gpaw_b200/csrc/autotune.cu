@@ -5,8 +5,7 @@
 // how many bands go into one launch.  A plan (TunePlan, internal.h) fixes
 //   * the kernel form: one thread per point (the small-grid form) or the
 //     marching kernel, which streams planes along axis 0;
-//   * the marching tile: 32, 16 or 8 columns wide (radius <= 2; larger radii
-//     have the 32-wide tile only);
+//   * the marching tile (TILE_*, internal.h);
 //   * the axis-0 split: a target number of CTAs per SM, which sets how many
 //     planes each CTA marches through.
 // gfd_autotune_operator / gfd_autotune_transformer time every candidate
@@ -16,10 +15,10 @@
 // (floor(log2(bands))).  Every later launch with that key uses the plan;
 // launches without an entry keep the built-in rules.  The cache can be saved
 // to and loaded from a text file (GFD_TUNE_CACHE=<path> loads one on first
-// use).  The marching candidates give bit-identical results; the
-// one-thread-per-point form sums a stencil's terms in another order, so it
-// differs from them at the rounding level (well inside the 1e-13 relative
-// parity bound).
+// use).  star_kernel's tiles and the flex tile give bit-identical results; the
+// lane-pair and column-pair kernels and the one-thread-per-point form sum a
+// stencil's terms in other orders and differ at the rounding level (well inside
+// the 1e-13 relative parity bound).
 #include <atomic>
 #include <cerrno>
 #include <cmath>
@@ -44,7 +43,7 @@ std::once_flag g_env_once;
 // Set while an autotune run times one candidate on this thread.
 thread_local const TunePlan* t_force = nullptr;
 
-const int kCps[] = {1, 2, 4, 8};
+const int kCps[] = {1, 2, 3, 4, 6, 8, 12};
 
 int band_class(int64_t nin) {
   int c = 0;
@@ -270,7 +269,11 @@ extern "C" int gfd_autotune_operator(gfd_operator* op, int dtype, int mode, cons
   if (dtype == GFD_COMPLEX128 && op->R == 3 && imode == OP_APPLY) tiles.push_back(TILE_PAIR);
   if (dtype == GFD_COMPLEX128 && op->R <= 3) tiles.push_back(TILE_FLEX);
   if (!dtype_is_complex(dtype) && tile48r_eligible(op)) tiles.push_back(TILE_48R);
-  const std::vector<TunePlan> cands = march_candidates(tiles);
+  std::vector<TunePlan> cands = march_candidates(tiles);
+  // The one-axis kernels have neither tiles nor a split: one thread per point
+  // or marching is all there is to time.
+  if (imode == OP_APPLY && line_apply_axis(op, (int)dtype_size(dtype), nin) >= 0)
+    cands = {TunePlan{PLAN_DIRECT}, TunePlan{PLAN_MARCH}};
   const double* ph = dtype_is_complex(dtype) ? phase_cd : nullptr;
   TunePlan pick;
   st = time_candidates(cands, reps, s,

@@ -74,7 +74,7 @@ int num_sms();
 // three rows per lane pair, 32 columns by 12 rows).
 // TILE_FLEX: complex128, radius <= 3, star_flex_kernel (tile sides that fit the
 // grid).
-// TILE_48R: real bands, radius <= 3, 48 columns by 16 rows (48 x 4 threads, 4
+// TILE_48R: real bands of radius 3, 48 columns by 16 rows (48 x 4 threads, 4
 // rows each), where 48-column tiles pad axis 2 less than 32-column ones.
 enum {
   TILE_WIDE = 0,

@@ -361,9 +361,9 @@ GFD_API int gfd_poisson_batch_grouped(const gfd_poisson_batch* batch, int* group
  * after one untimed launch; the output buffer is overwritten) and cache the
  * fastest under (operation, dtype, mode, grid, radius or order, boundary
  * conditions, floor(log2(bands))).  Later launches with that key use it;
- * others keep the built-in rules.  Marching candidates give bit-identical
- * results; the one-thread-per-point form sums a stencil's terms in another
- * order (rounding-level differences).  Residual sweeps keep the built-in
+ * others keep the built-in rules.  Tiles 0 to 3, 6, 8 and 9 give bit-identical
+ * results; tiles 4, 5 and 7 and the one-thread-per-point form sum a stencil's
+ * terms in other orders (rounding-level differences).  Residual sweeps keep the built-in
  * rules.  Not allowed on a stream that is being captured.
  * Plans take effect at the next launch: a Poisson solver's or batch's
  * captured graph keeps the plans it was captured with
@@ -379,10 +379,10 @@ typedef struct gfd_tune_plan {
   int tile;         /* marching tile: 0 32 columns, 1 16, 2 8, 3 32 columns x 8 rows,
                        4 complex bands with re / im on lane pairs (radius <= 3),
                        5 the same for complex128 on full rows staged by TMA,
-                       6 complex128, 48 columns x 8 rows (axis-2 lengths that are
+                       6 complex bands, 48 columns x 8 rows (axis-2 lengths that are
                        multiples of 48), 7 complex128 apply of radius 3, two
-                       columns per lane pair, 8 real bands, 48 columns x 16 rows,
-                       9 complex128 up to radius 3, tile sides that fit the grid */
+                       columns per lane pair, 8 real bands of radius 3, 48 columns
+                       x 16 rows, 9 complex128 up to radius 3, tile sides that fit the grid */
   int ctas_per_sm;  /* axis-0 split target */
   double us;        /* measured time per launch, microseconds */
 } gfd_tune_plan;

@@ -50,7 +50,7 @@ def force(path, kind, dtype, mode, n, order, per, nbands, plan):
 
 
 def per_mask(pbc):
-    return sum(1 << c for c in range(3) if pbc[c])
+    return sum(1 << c for c in range(3) if np.ravel(pbc * np.ones(3, int))[c])
 
 
 @pytest.mark.parametrize('n', [1, 3])
@@ -284,3 +284,54 @@ def test_tile48_matches_oracle(cuda, plans, nn, N, pbc):
         r64[tile] = out.cpu().numpy()
     assert np.array_equal(r64[6], r64[0])
     assert rel_err(r64[6].astype(complex), ref) < 2e-6
+
+
+FITTED = [((7, 10, 9), 0), ((13, 33, 31), (1, 0, 1)), ((9, 95, 95), 0), ((8, 25, 64), 1),
+          ((12, 13, 70), (0, 1, 0)), ((10, 16, 47), 0)]
+
+
+@pytest.mark.parametrize('N,pbc', FITTED)
+@pytest.mark.parametrize('nn', [1, 2, 3])
+def test_forced_fitted_tiles(cuda, plans, nn, N, pbc):
+    """Plan tiles 7 (column pairs), 8 (real, 48 columns) and 9 (fitted sides)
+    on grids the built-in rules give other tiles: odd columns, rows not in threes,
+    zero boundaries, fewer columns or rows than a tile; several splits, apply and
+    apply with a potential, phases."""
+    import torch
+    from gpaw_b200.fd_operators import FDOperator
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    og = G.Grid(N, np.array(N) * 0.25, pbc)
+    gd = GridDescriptor(og.N_c, og.cell_cv, og.pbc_c)
+    c, o = G.laplace_stencil(og, -0.5, nn)
+    rng = np.random.default_rng(nn)
+    a = rng.standard_normal((3,) + tuple(og.n_c))
+    v = rng.uniform(-1, 1, tuple(og.n_c))
+    ph = G.bloch_phases(og, (0.25, -0.1, 0.3))
+    for x, p, tiles in ((a, None, (8,)), (a + 1j * a[::-1], ph, (7, 9))):
+        t = torch.from_numpy(x.copy()).to(cuda)
+        op = FDOperator(c, o, gd, t.dtype)
+        ref = K.fd_apply(c, o, og.pbc_c, x, p)
+        for tile in tiles:
+            for mode, want in ((0, ref), (3, ref + v * x)):
+                for cps in (1, 3, 12):
+                    force(plans / 'p.txt', 0, 0 if p is None else 1, mode, og.n_c, nn,
+                          per_mask(og.pbc_c), 3, (1, tile, cps))
+                    out = torch.full_like(t, float('nan'))
+                    if mode == 0:
+                        op.apply(t, out, p)
+                    else:
+                        op.apply_with_potential(t, out, torch.from_numpy(v).to(cuda), p)
+                    torch.cuda.synchronize()
+                    assert rel_err(out.cpu().numpy(), want) < TOL, (tile, mode, cps)
+
+
+def test_one_axis_plans(cuda, plans):
+    """The one-axis kernels have neither tiles nor a split: the tuner stores one
+    thread per point or the marching default for a gradient."""
+    from gpaw_b200 import autotune
+    from gpaw_b200.fd_operators import Gradient
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    gd = GridDescriptor((40, 44, 48), (10.0, 11.0, 12.0), 1)
+    for axis in range(3):
+        plan = autotune.tune_operator(Gradient(gd, axis, 1.0, 3, complex), nbands=8, reps=1)
+        assert plan['form'] == 'direct' or (plan['tile'], plan['ctas_per_sm']) == (32, 4)

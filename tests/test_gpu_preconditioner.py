@@ -58,6 +58,28 @@ def test_preconditioner_matches_oracle(cuda, tag, N, pbc, dtype, k, nb, nn):
     assert rel_err(o32.cpu().numpy().astype(ref.dtype), ref) < 2e-6
 
 
+@pytest.mark.parametrize('N,pbc,nb', [((36, 68, 100), 0, 11), ((36, 76, 84), (1, 0, 1), 12),
+                                      ((24, 96, 96), 1, 24)])
+def test_large_blocks(cuda, N, pbc, nb):
+    """Blocks whose two upper levels pass the one-thread-per-point size, on planes
+    that fixed tiles pad a lot and a little: the marching Jacobi and residual
+    sweeps of complex bands (fitted and fixed tiles), zero boundaries, phases."""
+    import torch
+    from gpaw_b200.fd_operators import Laplace
+    from gpaw_b200.grid_descriptor import GridDescriptor
+    from gpaw_b200.preconditioner import Preconditioner
+    og = G.Grid(N, np.array(N) * 0.2 / BOHR, pbc)
+    gd = GridDescriptor(og.N_c, og.cell_cv, og.pbc_c)
+    rng = np.random.default_rng(nb)
+    shape = (nb,) + tuple(og.n_c)
+    R = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    ph = G.bloch_phases(og, (0.2, -0.3, 0.1))
+    kin0 = Laplace(gd, -0.5, 3, complex)
+    ref = OraclePC(og, (kin0.coef_p, kin0.offset_pc))(R, ph)
+    out = Preconditioner(gd, kin0, complex, block=nb)(torch.from_numpy(R).to(cuda), KPoint(ph))
+    assert rel_err(out.cpu().numpy(), ref) < TOL
+
+
 def test_preconditioner_rejects_bad_input(cuda):
     import torch
     from gpaw_b200.fd_operators import Laplace

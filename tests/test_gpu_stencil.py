@@ -271,7 +271,7 @@ def test_fitted_tiles(cuda, N, pbc, n):
     """Band batches past the one-thread-per-point size on grids around the
     fitted tiles' edges (32, 48 and 64 columns, rows in twos and threes, one
     row or column over): apply and apply with a potential, real and phased
-    complex128, and the Jacobi sweep of one large grid."""
+    complex128, and Jacobi sweeps of one band of as many points."""
     import torch
     from gpaw_b200.fd_operators import FDOperator
     from gpaw_b200.grid_descriptor import GridDescriptor
@@ -292,6 +292,16 @@ def test_fitted_tiles(cuda, N, pbc, n):
         out.fill_(float('nan'))
         op.apply_with_potential(t, out, dev(v, cuda), p)
         assert rel_err(host(out), ref + v * x) < TOL
+    # the batch as one grid: its planes side by side along axis 0
+    M = (nb * N[0],) + N[1:]
+    args = (M, np.array(M) * 0.25, pbc)
+    c, o = G.laplace_stencil(G.Grid(*args), -0.5, n)
+    gd = GridDescriptor(*args)
+    phi, rho = (rng.standard_normal(tuple(gd.n_c)) for _ in range(2))
+    t = dev(phi, cuda)
+    FDOperator(c, o, gd).relax(2, t, dev(rho, cuda), 3, 0.7)
+    K.relax(2, c, o, gd.pbc_c, phi, rho, 3, 0.7)
+    assert rel_err(host(t), phi) < TOL
 
 
 @pytest.mark.parametrize('nb', [1, 3, 12])

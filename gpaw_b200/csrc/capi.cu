@@ -94,6 +94,11 @@ int march_ctas_per_sm() {
   return v;
 }
 
+bool march_ctas_given() {
+  static const bool v = getenv("GFD_MARCH_CTAS_PER_SM") != nullptr;
+  return v;
+}
+
 int zero_launch(int dtype, void* y, int64_t n, cudaStream_t s) {
   const int blocks = grid_for(n);
   if (dtype == GFD_FLOAT64)

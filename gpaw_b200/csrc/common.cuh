@@ -238,9 +238,11 @@ bool pdl_enabled();
 bool split_enabled();
 // Largest grid (points over all bands) for the one-thread-per-point kernels.
 long long direct_max_points();
-// CTAs per SM the marching kernels aim for when they split axis 0 into
-// chunks (GFD_MARCH_CTAS_PER_SM, default 4).
+// CTAs per SM the marching kernels aim for when they split axis 0 into chunks:
+// GFD_MARCH_CTAS_PER_SM, for all of them where it is given; else 4 for those that
+// do not count the rounds of their CTAs (march_split.h).
 int march_ctas_per_sm();
+bool march_ctas_given();
 
 // Launch with the programmatic-stream-serialisation attribute when enabled
 // (GFD_PDL=1 in the environment; off by default).

@@ -43,4 +43,13 @@ inline MarchSplit march_split(int n0, int R, int64_t tiles, int resident, int sm
   return best;
 }
 
+// The chunk count of a launch.  target > 0: that many CTAs per SM, of a launch
+// plan or set for the process, whatever the rounds; else by march_split.
+inline int march_chunks(int n0, int R, int64_t tiles, int resident, int sms, int target) {
+  if (target <= 0) return march_split(n0, R, tiles, resident, sms).chunks;
+  const int64_t want = (int64_t(target) * sms + tiles - 1) / tiles;
+  const int most = std::max(1, n0 / std::max(4, 2 * R));
+  return int(std::min<int64_t>(most, std::max<int64_t>(1, want)));
+}
+
 }  // namespace gfd

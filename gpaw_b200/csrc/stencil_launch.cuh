@@ -73,8 +73,15 @@ struct LaunchGeom {
   int64_t bands_per_launch;
 };
 
-// resident: CTAs per SM of the kernel where known (0: aim for march_ctas_per_sm()
-// without counting rounds); cps: a launch plan's target.
+// The target in CTAs per SM that a launch is split by: a plan's (cps), the
+// environment's, four for kernels whose CTAs per SM are not known (resident 0),
+// else none, the rounds are counted.
+inline int split_target(int cps, int resident) {
+  if (cps > 0) return cps;
+  return resident > 0 && !march_ctas_given() ? 0 : march_ctas_per_sm();
+}
+
+// resident: CTAs per SM of the kernel where known; cps: a launch plan's target.
 inline LaunchGeom star_geom(const gfd_operator* op, int tile, int64_t nin, int R, int cps = 0,
                             int resident = 0) {
   TileDims td = tile_dims(tile);
@@ -82,11 +89,8 @@ inline LaunchGeom star_geom(const gfd_operator* op, int tile, int64_t nin, int R
   int gx = (op->n[2] + td.BZ - 1) / td.BZ;
   int gy = (op->n[1] + td.BY - 1) / td.BY;
   int64_t tiles = (int64_t)gx * gy * std::max<int64_t>(nin, 1);
-  int64_t target = (int64_t)(cps > 0 ? cps : march_ctas_per_sm()) * num_sms();
-  int maxc = std::max(1, op->n[0] / std::max(4, 2 * R));
-  int nxc = (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles));
-  if (cps == 0 && resident > 0)
-    nxc = march_split(op->n[0], R, tiles, resident, num_sms()).chunks;
+  const int nxc =
+      march_chunks(op->n[0], R, tiles, resident, num_sms(), split_target(cps, resident));
   g.x_chunk = (op->n[0] + nxc - 1) / nxc;
   g.nxc = (op->n[0] + g.x_chunk - 1) / g.x_chunk;
   g.bands_per_launch = std::max<int64_t>(1, 65535 / g.nxc);
@@ -487,11 +491,8 @@ template <class F>
 int march_launches(const gfd_operator* op, int gx, int gy, int64_t nin, int cps, int resident,
                    StarParams<double>& p, F launch) {
   const int64_t tiles = (int64_t)gx * gy * nin;
-  const int maxc = std::max(1, op->n[0] / std::max(4, 2 * op->R));
-  const int64_t target = (int64_t)cps * num_sms();  // a launch plan's
   const int nxc =
-      cps > 0 ? (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles))
-              : march_split(op->n[0], op->R, tiles, resident, num_sms()).chunks;
+      march_chunks(op->n[0], op->R, tiles, resident, num_sms(), split_target(cps, resident));
   p.x_chunk = (op->n[0] + nxc - 1) / nxc;
   p.nxc = (op->n[0] + p.x_chunk - 1) / p.x_chunk;
   const int64_t per_launch = std::max<int64_t>(1, 65535 / p.nxc);
@@ -890,7 +891,8 @@ inline DirGeom dirs_geom(const gfd_operator* op, int resident, int64_t nin) {
   g.ty = (rows + kDirVY - 1) / kDirVY;
   g.gy = (op->n[1] + g.ty * kDirVY - 1) / (g.ty * kDirVY);
   const int64_t tiles = (int64_t)g.gx * g.gy * std::max<int64_t>(nin, 1);
-  const int nxc = march_split(op->n[0], R, tiles, resident, num_sms()).chunks;
+  const int nxc =
+      march_chunks(op->n[0], R, tiles, resident, num_sms(), split_target(0, resident));
   g.x_chunk = (op->n[0] + nxc - 1) / nxc;
   g.nxc = (op->n[0] + g.x_chunk - 1) / g.x_chunk;
   g.bands_per_launch = std::max<int64_t>(1, 65535 / g.nxc);

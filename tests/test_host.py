@@ -285,11 +285,13 @@ def test_march_split_counts_whole_rounds(tmp_path):
                    'extern "C" int split(int n0, int R, long long tiles, int res, int sms,\n'
                    '                     double* steps) {\n'
                    '  auto s = gfd::march_split(n0, R, tiles, res, sms);\n'
-                   '  *steps = s.steps;\n  return s.chunks;\n}\n')
+                   '  *steps = s.steps;\n  return s.chunks;\n}\n'
+                   'extern "C" int chunks(int n0, int R, long long tiles, int res, int target) {\n'
+                   '  return gfd::march_chunks(n0, R, tiles, res, 148, target);\n}\n')
     lib = tmp_path / 'split.so'
     subprocess.run(['g++', '-std=c++17', '-O1', '-shared', '-fPIC', '-I',
                     os.path.join(ROOT, 'gpaw_b200', 'csrc'), str(src), '-o', str(lib)], check=True)
-    f = ctypes.CDLL(str(lib)).split
+    f, chunks_of = ctypes.CDLL(str(lib)).split, ctypes.CDLL(str(lib)).chunks
 
     def split(n0, R, tiles, res, sms=148):
         steps = ctypes.c_double()
@@ -303,6 +305,10 @@ def test_march_split_counts_whole_rounds(tmp_path):
     assert split(66, 3, 296, 2)[0] == 1
     assert split(80, 3, 160, 2) == (3, 66.0)  # 480 CTAs in two rounds of 33 steps
     assert split(1, 3, 5, 2) == (1, 0.75 * 7)
+    # a target of CTAs per SM is taken as it is, with the rounds known or not
+    for res in (0, 2):
+        assert [chunks_of(66, 3, ctypes.c_longlong(300), res, t) for t in (1, 4, 64)] == [1, 2, 11]
+    assert chunks_of(66, 3, ctypes.c_longlong(300), 2, 0) == split(66, 3, 300, 2)[0]
     rng = np.random.default_rng(1)
     for _ in range(300):
         n0, R, res = int(rng.integers(1, 200)), int(rng.integers(1, 7)), int(rng.integers(1, 6))

@@ -523,7 +523,7 @@ inline StepCost c128_fixed_cost(int tile, int R) {
   return {us * (resident + 1) / resident, resident + 1};
 }
 // Bloch phases of axes 1 and 2 cost the pair kernel 63%, the others 39 to 47%.
-inline StepCost pair_cost(bool phases) { return {phases ? 1.38 : 1.18, 3}; }
+inline StepCost pair_cost(bool phases) { return {phases ? 1.30 : 1.11, 3}; }
 
 // The tile with the least time per plane.  Measured for 108^3 R = 3, 64 bands:
 // (36, 6) 692 us, (36, 7) 725, (54, 4) 796; 90 x 100: (50, 5) 430, (26, 9) and

@@ -59,14 +59,35 @@ def measured_peaks():
         return 6650.0, 'fallback'
 
 
-def ncu_traffic():
-    """Per-launch DRAM bytes of the headline kernel from the committed ncu
-    summary (profiles/star_kernel_c128_96.txt: a line 'traffic_bytes_per_launch: X')."""
-    path = os.path.join(ROOT, 'profiles', 'star_kernel_c128_96.txt')
+# Kernel of a launch plan of the headline apply (complex128, radius 3).
+PLAN_KERNELS = {'pair': 'star_pair_kernel', 'flex': 'star_flex_kernel<3>',
+                'split': 'star_split_kernel<cplx<double>, 3>',
+                'tma-split': 'star_tmasplit_kernel<3>',
+                '48x8': 'star_kernel<cplx<double>, 3>, 48 x 8 tile',
+                '32x8': 'star_kernel<cplx<double>, 3>, 32 x 8 tile',
+                32: 'star_kernel<cplx<double>, 3>, 32 x 16 tile'}
+
+
+def plan_kernel(plan):
+    if plan is None:
+        return 'built-in choice (no launch plan)'
+    if plan['form'] == 'direct':
+        return 'star_direct_kernel<cplx<double>, 3>'
+    return PLAN_KERNELS.get(plan['tile'], str(plan['tile']))
+
+
+def ncu_traffic(plan):
+    """Per-launch DRAM bytes of the plan's kernel from the committed ncu summary
+    (profiles/star_kernel_c128_96.txt: lines 'traffic_bytes_per_launch TILE: X'),
+    None where there is none for it."""
+    if plan is None or plan['form'] == 'direct':
+        return None
+    key = 'traffic_bytes_per_launch %s:' % plan['tile']
     try:
-        for line in open(path):
-            if line.startswith('traffic_bytes_per_launch:'):
-                return float(line.split(':', 1)[1])
+        with open(os.path.join(ROOT, 'profiles', 'star_kernel_c128_96.txt')) as f:
+            for line in f:
+                if line.startswith(key):
+                    return float(line[len(key):])
     except OSError:
         pass
     return None
@@ -807,7 +828,7 @@ def run_gpu_arm(args):
         var = stencil_variants_bench(gd, a, b, phase, min(args.steps, 20))
 
     peak, peak_kind = measured_peaks()
-    traffic = ncu_traffic()
+    traffic = ncu_traffic(plan) if nb == NBANDS else None
     line = {'metric': METRIC, 'value': value, 'unit': 'GB/s', 'n_gpus': world,
             'steps': args.steps, 'warmup': args.warmup, 'ms_per_step': ms_max,
             'higher_is_better': True, 'scaling': 'weak', 'vs_baseline': None,
@@ -816,9 +837,7 @@ def run_gpu_arm(args):
             'roofline': {'bound': 'hbm', 'achieved': kernel_gbs, 'peak': peak, 'unit': 'GB/s',
                          'frac': kernel_gbs / peak, 'peak_kind': peak_kind,
                          'traffic': traffic, 'algorithmic_bytes_per_launch': nbytes,
-                         'kernel': ('star_direct_kernel<cplx<double>,R=3>'
-                                    if plan and plan['form'] == 'direct'
-                                    else 'star_pair_kernel (complex128, R=3; 96^3)')},
+                         'kernel': plan_kernel(plan)},
             'launch_plan': plan,
             'check': check,
             'e2e': e2e,

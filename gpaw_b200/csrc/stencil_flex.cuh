@@ -9,7 +9,9 @@
 // row cells of a thread are reads at fixed offsets.  Two rows per thread hold 4R
 // complex partial sums: 128 registers, 16 warps per SM.  Cells outside a
 // zero-boundary axis are cleared once and never copied; planes outside it are
-// skipped.  The order of the sums is star_kernel's.
+// skipped.  The order of the sums is star_kernel's.  84 x 90 x 100, 16 bands:
+// 120 us, the L1 pipe at 83%, short-scoreboard stalls 3.1 per issue: shared
+// reads and their latency bound it.
 #pragma once
 
 #include "common.cuh"

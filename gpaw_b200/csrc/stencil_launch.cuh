@@ -163,26 +163,26 @@ constexpr int kMaxComplexRelaxR = 3;
 
 // The short tile exists for complex128 apply (and apply with a potential)
 // up to radius 4 (beyond, its 2R + 1 partial sums per row do not fit the
-// registers of three CTAs per SM).  It is the built-in choice for those
-// launches where the 48-column tile below does not apply: on B200 (the
-// 512-band 96^3 Laplace, one box) it measured 3730 GB/s at four CTAs of 128
-// threads per SM, against 3120 for the 32 x 16 tile, 3100 for the lane-pair
-// kernel and 3270 for its TMA-staged form; three CTAs per SM with up to 170
-// registers took it to 3934.
+// registers of three CTAs per SM): the built-in choice at radius 4 where the
+// 48-column tile below does not apply, and up to radius 3 where c128_tile()
+// prices it lowest.  On the 512-band 96^3 Laplace (one box) it measured 3730
+// GB/s at four CTAs of 128 threads per SM, against 3120 for the 32 x 16 tile,
+// 3100 for the lane-pair kernel and 3270 for its TMA-staged form; three CTAs
+// per SM with up to 170 registers took it to 3934.
 constexpr int kMaxShortR = 4;
 template <class V, int R, int MODE>
 constexpr bool has_short_tile() {
   return sizeof(V) >= 16 && (MODE == MODE_APPLY || MODE == MODE_POTENTIAL) && R <= kMaxShortR;
 }
 // The 48-column tile: complex bands (complex128 and complex64), the same
-// launches; the built-in choice for both where axis 2 is a multiple of 48.
+// launches, where axis 2 is a multiple of 48: complex64's built-in choice, and
+// complex128's as for the short tile.
 template <class V, int R, int MODE>
 constexpr bool has_tile48() {
   return vt<V>::NC == 2 && (MODE == MODE_APPLY || MODE == MODE_POTENTIAL) && R <= kMaxShortR;
 }
-// The 48-column tile (TILE_48) covers the same launches where axis 2 is a
-// multiple of 48 and is then the built-in choice: 48 x 4 threads with 2
-// rows each, two CTAs per SM.  On the 512-band 96^3 Laplace it measured
+// 48 x 4 threads with 2 rows each, two CTAs per SM.  On the 512-band 96^3
+// Laplace the 48-column tile measured
 // 4010-4099 GB/s against 3730-3826 for the short tile at 4 CTAs per SM
 // (3934 at 3)
 // (apply with a potential: 3610-3750 against 3260-3380).  A 96-column tile
@@ -755,10 +755,11 @@ int launch_star_typed(const gfd_operator* op, int mode, const void* in, void* ou
       return star_tma_dispatch(op, vin, vout, nin, p, g, s);
     }
   }
-  // Radii above 2 have the wide tile only (and the short one for complex128
-  // apply); complex bands up to radius 3 have the lane-pair tile, their
-  // built-in choice wherever the wide tile would be picked.  Any other plan
-  // tile falls back to the built-in choice, so the geometry always matches
+  // Built-in choices: the wide tile (narrow ones for short rows of radius 1 and
+  // 2); complex applies the short or the 48-column tile, complex128 up to radius
+  // 3 by c128_tile(); real bands of radius 3 the 48-column tile where it pays.
+  // The lane-pair tiles come from plans only.  A plan's tile that a launch does
+  // not have falls back to the built-in choice, so the geometry always matches
   // the kernel launched.
   int tile = pick_tile(op);
   const bool split = split_eligible<V>(op);
@@ -1134,7 +1135,7 @@ int gs_split_sweeps(const gfd_operator* op, V* phi, const V* rho, int nsweeps, V
                     const StarParams<typename vt<V>::S>& p, cudaStream_t s) {
   const int n = (int)p.band, NC = R + 1;
   const int nq = p.n0 * p.n1 * gs_row_slots(p.n2, NC);
-  const int cap = 148 * 16;
+  const int cap = 16 * num_sms();
   const int nb = std::min((n + 255) / 256, cap), qb = std::min((nq + 255) / 256, cap);
   launch_k(gs_split_kernel<V, R + 1>, nb, 256, 0, s, phi, copy, p.n2, n, 1);
   for (int sw = 0; sw < nsweeps; sw++)

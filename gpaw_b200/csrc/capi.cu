@@ -284,10 +284,14 @@ extern "C" int gfd_density_interpolate(gfd_transformer* tr, const double* nt_sG,
                                      sizeof(double) * (kRedBlocks + 1), s),
                        "scratch of a reduction")))
     return st;
-  if (n < 2000000000)  // the last step of the loop stays below 2^31
-    launch_k(interp_sum_kernel<int>, blocks, kRedThreads, 0, s, nt_sG, (int)n, q, buf);
+  bool whole = true;
+  for (int c = 0; c < 3; c++)
+    if (q.per[c] && q.nf[c] != 2 * q.n[c]) whole = false;
+  if (whole && n < 2000000000)  // the last step of the loop stays below 2^31
+    launch_k(interp_sum_kernel<int, true>, blocks, kRedThreads, 0, s, nt_sG, (int)n, q, buf);
   else
-    launch_k(interp_sum_kernel<long long>, blocks, kRedThreads, 0, s, nt_sG, (long long)n, q, buf);
+    launch_k(interp_sum_kernel<long long, false>, blocks, kRedThreads, 0, s, nt_sG, (long long)n,
+             q, buf);
   st = check_launch("interp_sum_kernel");
   if (!st) st = final_sum_launch(buf, blocks, dv_fine, buf + kRedBlocks, s);
   if (!st)

@@ -81,29 +81,32 @@ struct InterpSum {
   int nn;
   double w[4];              // Lagrange weights by distance
 };
-__device__ __forceinline__ double interp_weight(const InterpSum& p, int a, int c) {
+// Weight of the coarse point at fine position f in the fine points that there are.
+__device__ __forceinline__ double interp_weight_at(const InterpSum& p, int a, int f) {
   const int nn = p.nn, nf = p.nf[a];
-  if (p.per[a] && nf == 2 * p.n[a]) return 2.0;  // one whole period
-  double s = 0.0;
-  // Other fine sizes on a periodic axis: every image of the point that reaches
-  // the fine points (the halo is one period wide at most).
-  for (int image = p.per[a] ? -1 : 0; image <= (p.per[a] ? 1 : 0); image++) {
-    const int f = 2 * (c + image * p.n[a]) + p.shift[a];
-    if (f - 2 * nn + 1 >= 0 && f + 2 * nn - 1 < nf) {
-      s += 2.0;
-      continue;
-    }
-    s += f >= 0 && f < nf ? 1.0 : 0.0;
-    for (int k = 0; k < nn; k++) {
-      const int hi = f + 2 * k + 1, lo = f - 2 * k - 1;
-      if (hi >= 0 && hi < nf) s += p.w[k];
-      if (lo >= 0 && lo < nf) s += p.w[k];
-    }
+  if (f - 2 * nn + 1 >= 0 && f + 2 * nn - 1 < nf) return 2.0;
+  double s = f >= 0 && f < nf ? 1.0 : 0.0;
+  for (int k = 0; k < nn; k++) {
+    const int hi = f + 2 * k + 1, lo = f - 2 * k - 1;
+    if (hi >= 0 && hi < nf) s += p.w[k];
+    if (lo >= 0 && lo < nf) s += p.w[k];
   }
   return s;
 }
+// WHOLE: periodic axes hold one whole period of fine points.  Otherwise every
+// image of the point that reaches the fine points counts (the halo is one period
+// wide at most).
+template <bool WHOLE>
+__device__ __forceinline__ double interp_weight(const InterpSum& p, int a, int c) {
+  const int f = 2 * c + p.shift[a];
+  if (!p.per[a]) return interp_weight_at(p, a, f);
+  if constexpr (WHOLE) return 2.0;
+  double s = 0.0;
+  for (int image = -1; image <= 1; image++) s += interp_weight_at(p, a, f + 2 * image * p.n[a]);
+  return s;
+}
 // I: index type that holds total.
-template <class I>
+template <class I, bool WHOLE>
 __global__ void __launch_bounds__(kRedThreads) interp_sum_kernel(
     const double* __restrict__ a, I total, const InterpSum p, double* __restrict__ partials) {
   pdl_enter();
@@ -114,7 +117,8 @@ __global__ void __launch_bounds__(kRedThreads) interp_sum_kernel(
   for (I i = I(blockIdx.x) * kRedThreads + threadIdx.x; i < total; i += step) {
     const I g = i % band, row = g / p.n[2];
     const int z = int(g - row * p.n[2]), x = int(row / p.n[1]), y = int(row - I(x) * p.n[1]);
-    s += a[i] * (interp_weight(p, 0, x) * interp_weight(p, 1, y) * interp_weight(p, 2, z));
+    s += a[i] * (interp_weight<WHOLE>(p, 0, x) * interp_weight<WHOLE>(p, 1, y) *
+                 interp_weight<WHOLE>(p, 2, z));
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;

@@ -353,7 +353,9 @@ restrict_kernel(const V* __restrict__ in, V* __restrict__ out,
 // ---------------------------------------------------------------------------
 // SUB: out = base - interpolated value (the multigrid correction
 // phi -= interpolate(e), in place when base == out).
-template <class V, int NN, int BZF, int TYF, int VYF, bool SUB>
+// TOTAL: the factor comes from p.total (the renormalised density; a form of its
+// own: carried in a register by all, it cost complex64 nn = 2 12%).
+template <class V, int NN, int BZF, int TYF, int VYF, bool SUB, bool TOTAL>
 __global__ void __launch_bounds__(BZF * TYF)
 interp_kernel(const V* __restrict__ in, V* out, const V* base,
               const TrParams<typename vt<V>::S> p) {
@@ -374,7 +376,7 @@ interp_kernel(const V* __restrict__ in, V* out, const V* base,
   const int X0 = xc * p.x_chunk, X1 = min(p.no0, X0 + p.x_chunk);
   const long long plane_in = (long long)p.ni1 * p.ni2;
   const long long plane_out = (long long)p.no1 * p.no2;
-  const S osc = out_factor(p);
+  [[maybe_unused]] const S factor = TOTAL ? out_factor(p) : S(1);
   const V* inb = in + bnd * p.band_in;
   V* outb = out + bnd * p.band_out;
   const V* baseb = SUB ? base + bnd * p.band_out : nullptr;
@@ -480,7 +482,8 @@ interp_kernel(const V* __restrict__ in, V* out, const V* base,
           if (y < p.no1 && z < p.no2) {
             V v = par ? ip_tap<NN, V>([&](int o) { return q[j][NN - 1 + o]; }) : q[j][NN - 1];
             const long long o = X * plane_out + (long long)y * p.no2 + z;
-            if (osc != S(1)) v = vmul(osc, v);
+            if constexpr (TOTAL) v = vmul(factor, v);
+            else if (p.out_scale != S(1)) v = vmul(p.out_scale, v);
             if constexpr (SUB) v = vsub(baseb[o], v);
             stcs(outb + o, v);
           }

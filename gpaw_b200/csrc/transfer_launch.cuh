@@ -4,6 +4,7 @@
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 
 #include "internal.h"
 #include "transfer.cuh"
@@ -56,8 +57,16 @@ int interp_go(const gfd_transformer* tr, const V* in, V* out, const V* base, int
   int nxc = (int)std::min<int64_t>(maxc, std::max<int64_t>(1, (target + tiles - 1) / tiles));
   p.x_chunk = (tr->nout[0] + nxc - 1) / nxc;
   p.nxc = (tr->nout[0] + p.x_chunk - 1) / p.x_chunk;
-  auto kern = base ? interp_kernel<V, NN, BZF, TYF, VYF, true>
-                   : interp_kernel<V, NN, BZF, TYF, VYF, false>;
+  auto kern = base ? interp_kernel<V, NN, BZF, TYF, VYF, true, false>
+                   : interp_kernel<V, NN, BZF, TYF, VYF, false, false>;
+  if (p.total) {
+    if constexpr (std::is_same_v<V, double>) {
+      if (base) return set_error(GFD_EINVAL, "a device factor is for plain interpolation");
+      kern = interp_kernel<V, NN, BZF, TYF, VYF, false, true>;
+    } else {
+      return set_error(GFD_EINVAL, "a device factor is for float64");
+    }
+  }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(interp_kernel)");
   const int64_t per_launch = std::max<int64_t>(1, 65535 / p.nxc);

@@ -654,26 +654,38 @@ __device__ __forceinline__ V restrict_point_at(const V* __restrict__ base, int X
   for (int j = 0; j < 2 * NN; j++) tz[j] = tr_map(fz - W + 2 * j, p.ni2, p.per2, 1);
   tz[2 * NN] = tr_map(fz, p.ni2, p.per2, 1);
   if constexpr (NN == 1) {
-    // All 27 loads first (see star_point_at).
-    TrTap tx[3], ty[3];
+    // The loads first (see star_point_at): all 27, or the nine of one plane at a
+    // time where 27 values need too many registers (complex128: 166, one block of
+    // 256 per SM).
+    TrTap ty[3];
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      tx[k] = tr_map(fx + k - 1, p.ni0, p.per0, p.ni1 * p.ni2);
-      ty[k] = tr_map(fy + k - 1, p.ni1, p.per1, p.ni2);
-    }
-    V c[3][3][3];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
+    for (int k = 0; k < 3; k++) ty[k] = tr_map(fy + k - 1, p.ni1, p.per1, p.ni2);
+    auto plane = [&](int ox) -> V {
+      const TrTap tx = tr_map(fx + ox, p.ni0, p.per0, p.ni1 * p.ni2);
+      V c[3][3];
 #pragma unroll
       for (int j = 0; j < 3; j++)
 #pragma unroll
-        for (int k = 0; k < 3; k++)
-          c[i][j][k] = tr_fetch<LD>(base, tx[i], ty[j], tz[k == 1 ? 2 : k >> 1], p);
-    V r = rst_tap<1, V>([&](int ox) {
+        for (int k = 0; k < 3; k++) c[j][k] = tr_fetch<LD>(base, tx, ty[j], tz[k == 1 ? 2 : k >> 1], p);
       return rst_tap<1, V>([&](int oy) {
-        return rst_tap<1, V>([&](int oz) { return c[ox + 1][oy + 1][oz + 1]; });
+        return rst_tap<1, V>([&](int oz) { return c[oy + 1][oz + 1]; });
       });
-    });
+    };
+    V below = vzero<V>(), own = vzero<V>(), above = vzero<V>();
+    if constexpr (sizeof(V) >= 16) {
+#pragma unroll 1
+      for (int i = -1; i <= 1; i++) {
+        const V v = plane(i);
+        if (i < 0) below = v;
+        else if (i == 0) own = v;
+        else above = v;
+      }
+    } else {
+      below = plane(-1);
+      own = plane(0);
+      above = plane(1);
+    }
+    V r = rst_tap<1, V>([&](int o) { return o == 0 ? own : o < 0 ? below : above; });
     if (p.out_scale != typename vt<V>::S(1)) r = vmul(p.out_scale, r);
     return r;
   }

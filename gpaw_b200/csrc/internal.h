@@ -107,20 +107,21 @@ inline int line_axis(const gfd_operator* op) {
 }
 // The axis of an apply that the one-axis kernels take past the
 // one-thread-per-point size (bytes: size of a value), or -1.  Rows past 1024
-// points stay with star_kernel, and so do float32 rows of radius 1 (radius 2: of
-// a zero-boundary axis) in launches past 12 million points whose planes
-// star_kernel pads to less than 1.5 times their points: 30 of those took 1.16
-// times as long with the one-axis kernel (up to 1.43), 160 others 0.8.
+// points stay with star_kernel.  So do, in launches past 12 million points whose
+// planes star_kernel pads to less than 1.5 times their points,
+//  * float32 rows of radius 1 (radius 2: of a zero-boundary axis): 30 of those
+//    took 1.16 times as long with the one-axis kernel (up to 1.43), 160 others 0.8;
+//  * complex bands of radius 1 along a zero-boundary axis 1: six of those took
+//    1.04 to 1.21 times as long, periodic ones 0.85.
 inline int line_apply_axis(const gfd_operator* op, int bytes, int64_t nin) {
   const int axis = line_axis(op);
-  if (axis < 2) return axis;
   const int64_t n1 = op->n[1], n2 = op->n[2];
-  if (n2 > 1024) return -1;
+  if (axis < 1 || (axis == 2 && n2 > 1024)) return axis < 1 ? axis : -1;
   const bool padded = ((n1 + 15) / 16 * 16) * ((n2 + 31) / 32 * 32) * 2 >= n1 * n2 * 3;
-  return bytes == 4 && (op->R == 1 || (op->R == 2 && !op->per[2])) && !padded &&
-                 op->n[0] * n1 * n2 * nin > 12000000
-             ? -1
-             : axis;
+  if (padded || op->n[0] * n1 * n2 * nin <= 12000000) return axis;
+  const bool zero = !op->per[axis];
+  if (axis == 2) return bytes == 4 && (op->R == 1 || (op->R == 2 && zero)) ? -1 : axis;
+  return !op->real && op->R == 1 && zero ? -1 : axis;
 }
 enum { PLAN_DIRECT = 0, PLAN_MARCH = 1 };               // one thread per point / marching
 enum { TK_STAR = 0, TK_RESTRICT = 1, TK_INTERP = 2 };

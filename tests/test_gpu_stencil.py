@@ -473,22 +473,28 @@ def test_one_axis_stencils(cuda, N, pbc, axis, n):
 
 
 @pytest.mark.parametrize('pbc', [0, 1])
-@pytest.mark.parametrize('n', [1, 2, 3])
-def test_large_float32_rows(cuda, pbc, n):
-    """float32 gradients along axis 2 on either side of the launch size from
-    which radii 1 and 2 stay with the three-axis kernel; the FP32 bound of 2e-6."""
+@pytest.mark.parametrize('axis,n,dtype', [(2, 1, np.float32), (2, 2, np.float32),
+                                          (2, 3, np.float32), (1, 1, np.complex64)])
+def test_large_one_axis_launches(cuda, pbc, axis, n, dtype):
+    """Gradients on either side of the launch size from which float32 rows and
+    complex axis 1 of radius 1 (2) stay with the three-axis kernel; the FP32 bound
+    of 2e-6."""
     import torch
     from gpaw_b200.fd_operators import Gradient
     from gpaw_b200.grid_descriptor import GridDescriptor
     gd = GridDescriptor((33, 65, 97), (8.0, 16.0, 24.0), pbc)
-    op = Gradient(gd, 2, 1.0, n, np.float32)
+    op = Gradient(gd, axis, 1.0, n, dtype)
     rng = np.random.default_rng(n)
     for nb in (2, 66):
-        a = rng.standard_normal((nb,) + tuple(gd.n_c)).astype(np.float32)
+        a = rng.standard_normal((nb,) + tuple(gd.n_c)).astype(dtype)
+        if dtype is np.complex64:
+            a = a + np.complex64(1j) * a[::-1]
+        wide = complex if dtype is np.complex64 else float
         out = torch.full_like(dev(a, cuda), float('nan'))
         op.apply(dev(a, cuda), out)
-        ref = K.fd_apply(op.coef_p, op.offset_pc, gd.pbc_c, a.astype(float), nthreads=8)
-        assert rel_err(host(out).astype(float), ref) < 2e-6
+        ref = K.fd_apply(op.coef_p, op.offset_pc, gd.pbc_c, a.astype(wide),
+                         np.ones((3, 2), complex) if wide is complex else None, nthreads=8)
+        assert rel_err(host(out).astype(wide), ref) < 2e-6
 
 
 BLOCKED_SHAPES = [((24, 16, 33), 1), ((40, 20, 36), 1), ((40, 20, 36), 0), ((17, 18, 40), (0, 1, 1)),

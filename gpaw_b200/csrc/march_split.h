@@ -3,9 +3,9 @@
 //
 // A CTA of a marching kernel takes planes + 2R steps for a chunk of `planes`
 // planes.  The chip runs whole CTAs, `resident` per SM at a time, so a launch
-// of 300 CTAs on 296 slots is two rounds, not 1.01.  Fitted to 13000 launches
+// of 300 CTAs on 296 slots is two rounds, not 1.01.  Fitted to 34000 timed launches
 // (complex128, float64 and float32, radius 1 to 3, grids of 24 to 144 points a
-// side, 1 to 64 bands, every split; 6 to 9% rms): the steps cost the same
+// side, 1 to 64 bands, every split; 5 to 10% rms): the steps cost the same
 // throughout, and a last round that puts k of the `resident` CTAs on an SM costs
 // 1/2 + k / (2 resident) of a full one, half of it being latency.  Priced by a
 // fraction of a round instead, 30 bands of 66^3 took 144 steps where 112 do.

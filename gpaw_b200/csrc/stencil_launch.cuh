@@ -504,7 +504,7 @@ int march_launches(const gfd_operator* op, int gx, int gy, int64_t nin, int cps,
 }
 
 // Time of one plane step of a CTA with its SM full, in microseconds, and the
-// CTAs that an SM holds (registers).  Fitted to 22000 launches of the four
+// CTAs that an SM holds (registers).  Fitted to 27000 timed launches of the four
 // kernels (grids of 24 to 144 points a side, 1 to 64 bands, every axis-0 split,
 // zero and periodic boundaries; 7 to 10% rms) with march_split.h's rounds.  A
 // potential adds 11% to each.

@@ -467,12 +467,14 @@ extern "C" int gfd_operator_relax(gfd_operator* op, int dtype, int relax_method,
     return set_error(GFD_EINVAL, "relaxation needs the diagonal (zero offset) as coefs[0]");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t bytes = (size_t)op->n[0] * op->n[1] * op->n[2] * dtype_size(dtype);
+  // Zero-boundary Gauss-Seidel does not need the operator's scratch grid: calls
+  // from several threads, the first ones among them, leave it alone.
+  if (relax_method == GFD_RELAX_GS && !op->per[0] && !op->per[1] && !op->per[2])
+    return gs_sweeps_own_copy(op, dtype, func, source, nrelax, bytes, s);
   int st = ensure_scratch(op, bytes);
   if (st) return st;
   if (relax_method == GFD_RELAX_GS)
-    return op->per[0] || op->per[1] || op->per[2]
-               ? op_gs_sweeps(op, dtype, func, source, nrelax, op->scratch, s)
-               : gs_sweeps_own_copy(op, dtype, func, source, nrelax, bytes, s);
+    return op_gs_sweeps(op, dtype, func, source, nrelax, op->scratch, s);
   // Weighted Jacobi with w = 0 leaves func unchanged.
   if (w == 0.0) return GFD_OK;
   // Weighted Jacobi: ping-pong between func and the scratch grid.

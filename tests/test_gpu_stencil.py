@@ -229,8 +229,10 @@ def test_colour_split_gauss_seidel(cuda, N, nn):
 
 def test_overlapping_gauss_seidel(cuda):
     """Zero-boundary Gauss-Seidel calls through one operator on two streams at a
-    time leave each other's arrays alone; a call that is being captured takes
-    no memory.  Colour passes are deterministic: the bits of a lone call."""
+    time, and from two threads whose calls are its first, leave each other's
+    arrays alone; a call that is being captured takes no memory.  Colour passes are
+    deterministic: the bits of a lone call."""
+    import threading
     import torch
     from gpaw_b200.fd_operators import FDOperator
     from gpaw_b200.grid_descriptor import GridDescriptor
@@ -241,6 +243,7 @@ def test_overlapping_gauss_seidel(cuda):
     phi = [torch.randn(tuple(gd.n_c), dtype=torch.float64, device=cuda) for _ in range(2)]
     rho = [torch.randn_like(p) for p in phi]
     alone = [p.clone() for p in phi]
+    threaded = [p.clone() for p in phi]
     for p, r in zip(alone, rho):
         op.relax(1, p, r, 20)
         torch.cuda.synchronize()
@@ -252,6 +255,19 @@ def test_overlapping_gauss_seidel(cuda):
             op.relax(1, p, r, 20)
     torch.cuda.synchronize()
     assert all(torch.equal(p, a) for p, a in zip(phi, alone))
+    fresh = FDOperator(c, o, gd, float)
+
+    def work(s, p, r):
+        with torch.cuda.stream(s):
+            fresh.relax(1, p, r, 20)
+
+    threads = [threading.Thread(target=work, args=a) for a in zip(streams, threaded, rho)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert all(torch.equal(p, a) for p, a in zip(threaded, alone))
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         op.relax(1, graph_phi, rho[0], 20)

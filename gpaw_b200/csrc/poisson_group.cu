@@ -614,11 +614,12 @@ int group_capture_body(PoissonGroup* G, cudaStream_t cs, cudaGraph_t body,
 
 // Solvers whose level-0 grid has at most GFD_GROUP_MAX_POINTS points join
 // groups (default 32768, about 32^3).  Measured on B200, grouping beats
-// graph branches for many small grids (128 solves of 32^3: 10.3K against
-// 7.5K Gauss-Seidel solves/s) and loses from about 40^3 up (64 solves of
-// 48^3: 4.6K against 5.0K), where the branches' concurrent kernels already
-// fill the GPU and the queue's per-tile barriers cost more than the
-// launches they save.  Up to the one-thread-per-point limit of the solve
+// graph branches for many small grids (128 solves of 32^3: 13.2K against
+// 7.5K Gauss-Seidel solves/s; 64 of 48^3: 6.5K against 6.1K) and loses on
+// mixes of larger ones (8 each of 48, 64, 80, 96^3: 2.3K against 3.0K),
+// where the branches' concurrent kernels already fill the GPU and the
+// queue's per-tile barriers cost more than the launches they save.  The
+// line is kept well below that crossover.  Up to the one-thread-per-point limit of the solve
 // alone (300K points), a grouped solve computes exactly what it computes
 // alone.
 bool group_eligible(const gfd_poisson* ps) {
